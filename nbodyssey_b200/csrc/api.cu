@@ -181,16 +181,15 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
   return NB_OK;
 }
 
-int ws_reserve_energy(Workspace& w, int n, int blocks, int jsplit) {
+int ws_reserve_energy(Workspace& w, int blocks, int parts) {
   NB_TRY(ws_basic(w));
   if (blocks * 5 > w.epart_cap) {
     NB_TRY(dalloc(&w.epart, (size_t)blocks * 5));
     w.epart_cap = blocks * 5;
   }
-  size_t need = (size_t)jsplit * n;
-  if (need > (size_t)w.ephi_cap) {
-    NB_TRY(dalloc(&w.ephi, need));
-    w.ephi_cap = (int)need;
+  if (parts > w.ephi_cap) {
+    NB_TRY(dalloc(&w.ephi, (size_t)parts));
+    w.ephi_cap = parts;
   }
   return NB_OK;
 }

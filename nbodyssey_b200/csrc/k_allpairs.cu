@@ -496,60 +496,127 @@ int launch_ens_allpairs(const EnsArgs& e, const EnsAllPairs& ap, cudaStream_t st
 }
 
 // ---------------------------------------------------------------------------
-// Energy.  PE = -1/2 G sum_i m_i (phi_i - self_i), phi_i = sum_j m_j
-// rsqrt(r_ij^2 + eps^2) including j == i (removed again with the same float
-// rsqrt(eps^2) the loop used for it).  Pair math in FP32, per-tile partial
-// sums converted to FP64; KE, PE and momentum reduced in FP64 in a fixed
-// order (block partials, then the last block).
+// Energy.  PE = -G sum_{i<j} m_i m_j rsqrt(r_ij^2 + eps^2), each unordered pair
+// once.  A CTA holds a tile of kEThreads x K particles (K per thread) and runs
+// over its chunk of the partners from the tile's own start on: partners past
+// the tile count once; the tile's own particles are summed in both orders with
+// the self term, so that part is halved and the self term (the same float
+// rsqrt(eps^2) the loop used) removed.  Pair math in FP32, two partners per
+// packed instruction; each 256-partner sum is added in FP64, and KE, PE and
+// momentum are reduced in FP64 in a fixed order (block partials, then the last
+// block).
+//
+// Bound: 8 packed FP32 operations and 2 MUFU rsqrt per two pairs, which fill
+// the FMA pipe (64 packed lanes a cycle and SM) and the MUFU unit (16) alike:
+// 1.09 ms for the 5e9 pairs of n = 100,000 on 148 SMs at 1.93 GHz.  Measured
+// 1.40 ms a call there; the form that took every pair in both orders with
+// scalar FP32, 3.93 ms.
 // ---------------------------------------------------------------------------
-constexpr int kEThreads = 256;
-constexpr int kETile = 256;
+constexpr int kEThreads = 128;
+constexpr int kETile = 256;      // partners staged together
+constexpr int kEReduceThreads = 256;
 
-__global__ void __launch_bounds__(kEThreads) k_energy_phi(
+template <int K>
+__global__ void __launch_bounds__(kEThreads) k_energy_pairs(
     const float4* __restrict__ pos, int n, float eps2, int jchunk,
-    double* __restrict__ phi_part) {
-  __shared__ float4 s_src[kETile];
-  const int i = blockIdx.x * kEThreads + threadIdx.x;
-  const float4 bi = pos[i < n ? i : n - 1];
-  const int j0 = blockIdx.y * jchunk;
-  const int j1 = min(j0 + jchunk, n);
-  double phi = 0.0;
-  for (int jt = j0; jt < j1; jt += kETile) {
-    int j = jt + threadIdx.x;
-    s_src[threadIdx.x] = j < j1 ? pos[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    float acc = 0.f;
-#pragma unroll 8
-    for (int q = 0; q < kETile; ++q) {
-      float4 s = s_src[q];
-      float dx = s.x - bi.x, dy = s.y - bi.y, dz = s.z - bi.z;
-      float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-      acc = fmaf(s.w, mufu_rsqrt(__fadd_rn(r2, eps2)), acc);
-    }
-    phi += (double)acc;
-    __syncthreads();
+    double* __restrict__ pe_part) {
+  __shared__ __align__(16) float s_src[kETile * 4];   // (x0,x1,y0,y1)(z0,z1,m0,m1) pairs
+  __shared__ double s_r[kEThreads / 32];
+  constexpr int T = kEThreads * K;
+  const int tid = threadIdx.x;
+  const int i0 = blockIdx.x * T;
+  const int j1 = min((int)(blockIdx.y + 1) * jchunk, n);
+  const int j0 = max((int)blockIdx.y * jchunk, i0);   // T is a multiple of kETile or divides it
+  f2 nx[K], ny[K], nz[K];
+  double once[K], own[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = i0 + k * kEThreads + tid;
+    const float4 p = pos[i < n ? i : n - 1];
+    nx[k] = pk2(-p.x, -p.x);
+    ny[k] = pk2(-p.y, -p.y);
+    nz[k] = pk2(-p.z, -p.z);
+    once[k] = own[k] = 0.0;
   }
-  if (i < n) phi_part[(size_t)blockIdx.y * n + i] = phi;
+  const f2 e2 = pk2(eps2, eps2);
+  for (int jt = j0; jt < j1;) {
+    // a stage never mixes the tile's own particles with later ones
+    const int je = min(jt < i0 + T ? min(jt + kETile, i0 + T) : jt + kETile, j1);
+    __syncthreads();   // the previous stage has been read
+    for (int k = tid; k < kETile; k += kEThreads) {
+      const float4 p = jt + k < je ? pos[jt + k] : make_float4(0.f, 0.f, 0.f, 0.f);
+      float* q = &s_src[(k >> 1) * 8 + (k & 1)];
+      q[0] = p.x; q[2] = p.y; q[4] = p.z; q[6] = p.w;
+    }
+    __syncthreads();
+    f2 acc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = 0ull;
+    const int pairs = (je - jt + 1) >> 1;
+    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(s_src);
+#pragma unroll 4
+    for (int q = 0; q < pairs; ++q) {
+      const ulonglong2 A = src[2 * q], B = src[2 * q + 1];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const f2 dx = add2(A.x, nx[k]), dy = add2(A.y, ny[k]), dz = add2(B.x, nz[k]);
+        // eps^2 last: seeding the chain with it saves an instruction but
+        // shifts the sum's rounding bias (2e-9 of PE at n = 100,000)
+        const f2 r2 = add2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), e2);
+        float r0, r1;
+        up2(r2, r0, r1);
+        acc[k] = fma2(B.y, pk2(mufu_rsqrt(r0), mufu_rsqrt(r1)), acc[k]);
+      }
+    }
+    const bool mine = jt < i0 + T;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      float u, v;
+      up2(acc[k], u, v);
+      const double s = (double)u + (double)v;
+      if (mine) own[k] += s;
+      else once[k] += s;
+    }
+    jt = je;
+  }
+  // the chunk that starts this tile's run over its own particles removes the
+  // self terms
+  const bool self = j0 == i0 && j0 < j1;
+  const float self_inv = mufu_rsqrt(eps2);
+  double pe = 0.0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = i0 + k * kEThreads + tid;
+    if (i >= n) continue;
+    const float m = pos[i].w;
+    const double s = self ? (double)__fmul_rn(m, self_inv) : 0.0;
+    pe += (double)m * (once[k] + 0.5 * (own[k] - s));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pe += __shfl_down_sync(0xffffffffu, pe, o);
+  if ((tid & 31) == 0) s_r[tid >> 5] = pe;
+  __syncthreads();
+  if (tid == 0) {
+    double v = 0.0;
+    for (int w = 0; w < kEThreads / 32; ++w) v += s_r[w];
+    pe_part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = v;
+  }
 }
 
-__global__ void __launch_bounds__(kEThreads) k_energy_reduce(
-    const float4* __restrict__ pos, const float4* __restrict__ vel, int n,
-    float eps2, float G, int jsplit, const double* __restrict__ phi_part,
+__global__ void __launch_bounds__(kEReduceThreads) k_energy_reduce(
+    const float4* __restrict__ pos, const float4* __restrict__ vel, int n, float G,
+    int nparts, const double* __restrict__ pe_part,
     double* __restrict__ epart, unsigned* ticket, double* out) {
-  __shared__ double s_r[kEThreads / 32][5];
+  __shared__ double s_r[kEReduceThreads / 32][5];
   __shared__ bool s_last;
   double r[5] = {0, 0, 0, 0, 0};   // KE, PE, Px, Py, Pz
-  const double self_inv = (double)mufu_rsqrt(eps2);
-  for (int i = blockIdx.x * kEThreads + threadIdx.x; i < n;
-       i += gridDim.x * kEThreads) {
-    float4 p = pos[i];
-    float4 v = vel[i];
-    double m = (double)p.w;
-    double phi = 0.0;
-    for (int js = 0; js < jsplit; ++js) phi += phi_part[(size_t)js * n + i];
-    double self = (double)__fmul_rn(p.w, (float)self_inv);
+  const int stride = gridDim.x * kEReduceThreads;
+  const int first = blockIdx.x * kEReduceThreads + threadIdx.x;
+  for (int i = first; i < nparts; i += stride) r[1] += pe_part[i];
+  for (int i = first; i < n; i += stride) {
+    const double m = (double)pos[i].w;
+    const float4 v = vel[i];
     r[0] += 0.5 * m * ((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z);
-    r[1] += m * (phi - self);
     r[2] += m * v.x;
     r[3] += m * v.y;
     r[4] += m * v.z;
@@ -563,7 +630,7 @@ __global__ void __launch_bounds__(kEThreads) k_energy_reduce(
   __syncthreads();
   if (threadIdx.x < 5) {
     double v = 0.0;
-    for (int w = 0; w < kEThreads / 32; ++w) v += s_r[w][threadIdx.x];
+    for (int w = 0; w < kEReduceThreads / 32; ++w) v += s_r[w][threadIdx.x];
     epart[blockIdx.x * 5 + threadIdx.x] = v;
   }
   __threadfence();
@@ -572,40 +639,52 @@ __global__ void __launch_bounds__(kEThreads) k_energy_reduce(
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  // the last block: warp c sums component c over the blocks, lane by lane in
+  // block order, then across the lanes
+  if (warp < 5) {
+    double t = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(&epart[b * 5 + warp]);
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) s_r[0][warp] = t;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    double t[5] = {0, 0, 0, 0, 0};
-    for (int b = 0; b < (int)gridDim.x; ++b)
-      for (int c = 0; c < 5; ++c) t[c] += __ldcg(&epart[b * 5 + c]);
-    double ke = t[0];
-    double pe = -0.5 * (double)G * t[1];
+    const double ke = s_r[0][0], pe = -(double)G * s_r[0][1];
     out[0] = ke + pe;
     out[1] = ke;
     out[2] = pe;
-    out[3] = t[2];
-    out[4] = t[3];
-    out[5] = t[4];
+    out[3] = s_r[0][2];
+    out[4] = s_r[0][3];
+    out[5] = s_r[0][4];
     *ticket = 0u;
   }
 }
 
+// Tiles of 512 particles (K = 4: four targets share each staged load) from
+// n = 16,384 on, where they give more than 500 half-empty-triangle CTAs of one
+// tile each; below, tiles of 128 keep the device's SMs supplied.
 int launch_energy(Workspace& w, int n, const float4* pos, const float4* vel,
                   float eps2, float G, cudaStream_t st) {
-  const int itiles = (n + kEThreads - 1) / kEThreads;
   const int sms = device_sm_count();
-  int js = (sms * 4 + itiles - 1) / itiles;
-  const int jt = (n + kETile - 1) / kETile;
+  const bool wide = n >= 16384;
+  const int tile = kEThreads * (wide ? 4 : 1);
+  const int itiles = (n + tile - 1) / tile;
+  // about 16 CTAs per SM over the triangle, chunks of whole 512s
+  int js = (32 * sms + itiles - 1) / itiles;
+  const int jt = (n + 511) / 512;
   if (js > jt) js = jt;
   if (js < 1) js = 1;
-  int jchunk = (jt + js - 1) / js * kETile;
+  const int jchunk = (jt + js - 1) / js * 512;
   js = (n + jchunk - 1) / jchunk;
-  int rblocks = (n + kEThreads - 1) / kEThreads;
+  int rblocks = (n + kEReduceThreads - 1) / kEReduceThreads;
   if (rblocks > 2 * sms) rblocks = 2 * sms;
-  NB_TRY(ws_reserve_energy(w, n, rblocks, js));
-  k_energy_phi<<<dim3(itiles, js), kEThreads, 0, st>>>(pos, n, eps2, jchunk,
-                                                        w.ephi);
+  NB_TRY(ws_reserve_energy(w, rblocks, itiles * js));
+  const dim3 grid(itiles, js);
+  if (wide) k_energy_pairs<4><<<grid, kEThreads, 0, st>>>(pos, n, eps2, jchunk, w.ephi);
+  else k_energy_pairs<1><<<grid, kEThreads, 0, st>>>(pos, n, eps2, jchunk, w.ephi);
   NB_CUDA(cudaGetLastError());
-  k_energy_reduce<<<rblocks, kEThreads, 0, st>>>(
-      pos, vel, n, eps2, G, js, w.ephi, w.epart, w.eticket, w.eout);
+  k_energy_reduce<<<rblocks, kEReduceThreads, 0, st>>>(
+      pos, vel, n, G, itiles * js, w.ephi, w.epart, w.eticket, w.eout);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
@@ -681,7 +760,7 @@ int warm_allpairs_kernels() {
                   k_allpairs_queue<128, 2>, k_allpairs_queue<128, 4>,
                   k_allpairs_queue<128, 8>, k_allpairs_queue<256, 2>,
                   k_allpairs_queue<256, 4>, k_allpairs_queue<256, 8>, k_ens_pack,
-                  k_pack_static, k_energy_phi, k_energy_reduce);
+                  k_pack_static, k_energy_pairs<1>, k_energy_pairs<4>, k_energy_reduce);
 }
 
 }  // namespace nb

@@ -125,7 +125,7 @@ struct Workspace {
   // energy
   double* epart = nullptr;        // per-block partials [blocks][6]
   int epart_cap = 0;
-  double* ephi = nullptr;         // j-split phi partials [jsplit][cap]
+  double* ephi = nullptr;         // potential-energy partials, one per CTA
   int ephi_cap = 0;
   double* eout = nullptr;         // [8]
   unsigned* eticket = nullptr;    // last-block ticket of the energy reduce
@@ -143,7 +143,7 @@ constexpr int kPrepMaxBlocks = 1024;
 int ws_reserve(Workspace& w, int n, int key_bits);
 struct APGeom;
 int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g);
-int ws_reserve_energy(Workspace& w, int n, int blocks, int jsplit);
+int ws_reserve_energy(Workspace& w, int blocks, int parts);
 void ws_free(Workspace& w);
 
 // ---------------------------------------------------------------------------
