@@ -2,6 +2,7 @@
 // handle, pipeline orchestration (eager or one captured CUDA graph per step),
 // phase timing, and the device-pointer drop-ins for compute_forces /
 // leapfrog_step / total_energy (src/forces.cuh:8, src/integrator.cuh:19-21).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -75,6 +76,7 @@ int warm_kernels() {
   NB_TRY(warm_lbvh_kernels());
   NB_TRY(warm_walk_kernels());
   NB_TRY(warm_allpairs_kernels());
+  NB_TRY(warm_allpairs_sym_kernels());
   NB_TRY(warm_fns(k_differ));
   done[dev] = true;
   return NB_OK;
@@ -160,6 +162,24 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   return NB_OK;
 }
 
+// Scratch of the pairs-once kernel: all rows of tiles up to 1 GiB, fewer when
+// that cannot be had (one row at least).
+static int ws_reserve_allpairs_sym(Workspace& w, int n) {
+  NB_TRY(ws_basic(w));
+  const size_t row = allpairs_sym_row_f4(n);
+  const size_t tiles = allpairs_sym_geometry(n).tiles;
+  size_t rows = std::max<size_t>(1, std::min(tiles, ((size_t)1 << 26) / row));
+  if ((size_t)w.part_cap >= rows * row) return NB_OK;
+  for (;; rows = (rows + 1) / 2) {
+    w.part_cap = 0;
+    const int rc = dalloc(&w.part, rows * row);
+    if (rc == NB_OK) break;
+    if (rows == 1) return rc;
+  }
+  w.part_cap = (int)(rows * row);
+  return NB_OK;
+}
+
 int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
   NB_TRY(ws_basic(w));
   int npad = (n + kSrcTile - 1) / kSrcTile * kSrcTile;
@@ -179,6 +199,11 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
     w.tickets_cap = itiles;
   }
   return NB_OK;
+}
+
+int ws_reserve_naive(Workspace& w, int n) {
+  if (allpairs_sym(n)) return ws_reserve_allpairs_sym(w, n);
+  return ws_reserve_allpairs(w, n, allpairs_geometry(n));
 }
 
 int ws_reserve_energy(Workspace& w, int blocks, int parts) {
@@ -290,7 +315,7 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   if (force == NB_FORCE_AUTO)
     force = resolve_force_tuned(force, a.n, std::sqrt(a.theta2), a.traverse);
   // workspace growth (allocation, host side) stays outside the timed region
-  if (force == NB_FORCE_NAIVE) NB_TRY(ws_reserve_allpairs(w, a.n, allpairs_geometry(a.n)));
+  if (force == NB_FORCE_NAIVE) NB_TRY(ws_reserve_naive(w, a.n));
   else if (a.n >= 2) NB_TRY(ws_reserve(w, a.n, a.key_bits));
   if (pm) NB_CUDA(cudaEventRecord(pm->start, st));
   if (force == NB_FORCE_BH && a.n < 2) {
@@ -300,7 +325,9 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
     return mark(pm, NB_PHASE_WALK, st);
   }
   if (force == NB_FORCE_NAIVE) {
-    NB_TRY(launch_prep(w, a, false, true, st));
+    // the pairs-once kernel reads the positions themselves: nothing to pack
+    const bool sym = allpairs_sym(a.n);
+    if (!sym || a.kick_drift) NB_TRY(launch_prep(w, a, false, !sym, st));
     if (a.after_prep) NB_CUDA(cudaEventRecord(a.after_prep, st));
     NB_TRY(mark(pm, NB_PHASE_PREP, st));
     NB_TRY(launch_allpairs(w, a, st));
@@ -510,7 +537,7 @@ static int sim_capture(nb_sim* s) {
   if (resolve_force(s->p, s->n) == NB_FORCE_BH)
     NB_TRY(ws_reserve(s->ws, s->n, s->p.key_bits));
   else
-    NB_TRY(ws_reserve_allpairs(s->ws, s->n, allpairs_geometry(s->n)));
+    NB_TRY(ws_reserve_naive(s->ws, s->n));
   cudaGraph_t g = nullptr;
   NB_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   int rc = sim_step_eager(s, nullptr);
@@ -622,7 +649,7 @@ int nb_sim_create(int n, const float* pos4, const float* vel4,
     if ((rc = ws_basic(s->ws)) != NB_OK) break;
     // the force module's workspace now, not inside the first (timed) call
     if (resolve_force(s->p, n) == NB_FORCE_NAIVE)
-      rc = ws_reserve_allpairs(s->ws, n, allpairs_geometry(n));
+      rc = ws_reserve_naive(s->ws, n);
     else if (n >= 2)
       rc = ws_reserve(s->ws, n, s->p.key_bits);
     if (rc != NB_OK) break;

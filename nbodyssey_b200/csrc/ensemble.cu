@@ -234,13 +234,14 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     if (rc != NB_OK) break;
     if ((rc = ens_alloc(h, &e.walk_ctr, 2)) != NB_OK) break;
     h->ap_pool_f4 = plan_ens_allpairs(sims.data(), nsims, nullptr, h->ap);
-    if (!h->ap.args.empty()) {
+    if (h->ap_pool_f4 > 0) {
       EnsAllPairs& ap = h->ap;
       if ((rc = ens_alloc(h, &ap.d_pool, h->ap_pool_f4)) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_args, ap.args.size())) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_items, ap.items.size())) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_src_off, (size_t)nsims)) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_counter, 6)) != NB_OK) break;
+      if ((rc = ens_alloc(h, &ap.sym.d_table, ap.sym.bytes())) != NB_OK) break;
     }
     {
       BuildRun* runs = nullptr;
@@ -292,7 +293,7 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     if (ce == cudaSuccess && h->ap.d_pool)
       ce = cudaMemsetAsync(h->ap.d_pool, 0, sizeof(float4) * h->ap_pool_f4, st);
     if (ce != cudaSuccess) { rc = set_error(NB_ERR_CUDA, cudaGetErrorString(ce)); break; }
-    if (!h->ap.args.empty() &&
+    if (h->ap_pool_f4 > 0 &&
         (rc = bind_ens_allpairs(h->ap, sims.data(), nsims, e, st)) != NB_OK) break;
     ce = cudaStreamSynchronize(st);
     if (ce != cudaSuccess) { rc = set_error(NB_ERR_CUDA, cudaGetErrorString(ce)); break; }
@@ -321,6 +322,7 @@ int nb_ensemble_kernels_per_step(const nb_ensemble* h, int* kernels) {
     for (int q = 0; q < 2; ++q) k += h->walk_items[q].empty() ? 0 : 1;
   }
   if (!h->ap.groups.empty()) k += 1 + (int)h->ap.groups.size();   // pack + queues
+  k += 2 * (int)h->ap.sym.passes.size();   // pairs-once items and their reduction
   *kernels = k;
   return NB_OK;
 }

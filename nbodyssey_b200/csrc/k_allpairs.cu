@@ -333,6 +333,9 @@ int launch_allpairs_geom(Workspace& w, const StepArgs& s, const APGeom& g,
 }
 
 int launch_allpairs(Workspace& w, const StepArgs& s, cudaStream_t st) {
+  if (allpairs_sym(s.n))
+    return launch_allpairs_sym(s.n, s.pos, s.acc, s.kick_after ? s.vel : nullptr, s.eps2, s.G,
+                               s.half_dt, w.part, (size_t)w.part_cap, st);
   return launch_allpairs_geom(w, s, allpairs_geometry(s.n), st);
 }
 
@@ -372,7 +375,15 @@ size_t ap_region_f4(int n) {
   const size_t npad = (size_t)(n + kSrcTile - 1) / kSrcTile * kSrcTile;
   const size_t part = g.jsplit > 1 ? (size_t)g.jsplit * n : 0;
   const size_t tick = ((size_t)g.itiles + 3) / 4;
-  return (npad + part + tick + 15) / 16 * 16;
+  size_t f4 = npad + part + tick;
+  if (allpairs_sym(n)) f4 = std::max(f4, allpairs_sym_row_f4(n));
+  return (f4 + 15) / 16 * 16;
+}
+
+size_t ap_region_whole_f4(int n) {
+  if (!allpairs_sym(n)) return ap_region_f4(n);
+  return std::max(ap_region_f4(n),
+                  (allpairs_sym_row_f4(n) * allpairs_sym_geometry(n).tiles + 15) / 16 * 16);
 }
 
 size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of,
@@ -384,6 +395,14 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
   ap.items.clear();
   ap.groups.clear();
   ap.src_off.assign(nsims, -1);
+  ap.sym.clear();
+  // the tables of the pairs-once simulations, whole when they may be
+  size_t whole = 0;
+  for (int s = 0; s < nsims; ++s)
+    if (sims[s].active && sims[s].force == NB_FORCE_NAIVE) whole += ap_region_whole_f4(sims[s].n);
+  auto size_of = [&](int n) {
+    return whole <= ((size_t)1 << 26) ? ap_region_whole_f4(n) : ap_region_f4(n);
+  };
   struct Pending { int a; APGeom g; };
   std::vector<Pending> todo;
   size_t next = 0, top = 0;
@@ -401,18 +420,24 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
     a.G = d.G;
     a.half_dt = d.half_dt;
     const size_t r = region_of ? region_of[s] : next;
-    next = r + ap_region_f4(d.n);
-    if (region_cap && ap_region_f4(d.n) > region_cap[s]) {   // the table changed
+    const size_t size = region_cap ? region_cap[s] : size_of(d.n);
+    if (ap_region_f4(d.n) > size) {   // the table changed
       if (too_small) ++*too_small;
       continue;
     }
+    next = r + size;
     top = std::max(top, next);
+    if (allpairs_sym(d.n)) {
+      ap.sym.add(s, d, r, size);
+      continue;
+    }
     ap.src_off[s] = (int)r;
     todo.push_back({(int)ap.args.size(), g});
     ap.args.push_back(a);
     ap.sim.push_back(s);
     ap.region.push_back(r);
   }
+  ap.sym.finish();
   // one group per launch shape; items longest chunks first
   for (int threads : {128, 256})
     for (int k : {2, 4, 8}) {
@@ -456,7 +481,7 @@ int bind_ens_allpairs(EnsAllPairs& ap, const SimDesc* sims, int nsims, const Ens
                             cudaMemcpyHostToDevice, st));
   NB_CUDA(cudaMemcpyAsync(ap.d_src_off, ap.src_off.data(), sizeof(int) * nsims,
                           cudaMemcpyHostToDevice, st));
-  return NB_OK;
+  return ap.sym.bind(sims, e, ap.d_pool, st);
 }
 
 template <int T, int K>
@@ -465,6 +490,7 @@ static void launch_queue(const APQueue& q, int grid, cudaStream_t st) {
 }
 
 int launch_ens_allpairs(const EnsArgs& e, const EnsAllPairs& ap, cudaStream_t st) {
+  NB_TRY(ap.sym.launch(e, st));
   if (ap.groups.empty()) return NB_OK;
   k_ens_pack<<<(e.nblocks * 32 + 255) / 256, 256, 0, st>>>(e, ap.d_src_off, ap.d_pool);
   NB_CUDA(cudaGetLastError());

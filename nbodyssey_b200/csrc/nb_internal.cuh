@@ -143,6 +143,8 @@ constexpr int kPrepMaxBlocks = 1024;
 int ws_reserve(Workspace& w, int n, int key_bits);
 struct APGeom;
 int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g);
+// all-pairs scratch of the kernel that n particles use
+int ws_reserve_naive(Workspace& w, int n);
 int ws_reserve_energy(Workspace& w, int blocks, int parts);
 void ws_free(Workspace& w);
 
@@ -314,6 +316,27 @@ bool allpairs_shape_compiled(int threads, int k);
 int launch_allpairs_geom(Workspace& w, const StepArgs& a, const APGeom& g,
                          cudaStream_t st);
 
+// All-pairs with each unordered pair evaluated once (k_allpairs_sym.cu): a
+// function of n alone (order of the sums included), whatever the tuning table.
+// A step of kSymMin particles takes 14.4 us against 20.5 with the tiled kernel;
+// below, batches of small simulations keep the tiled kernel's work queue, and
+// kSymMax bounds the tables that a batch's plan uploads.
+constexpr int kSymMin = 2048;
+constexpr int kSymMax = 1 << 20;
+bool allpairs_sym(int n);
+struct SymGeom {
+  int tile, chunk;      // targets and sources of a work item
+  int tiles, chunks;
+};
+SymGeom allpairs_sym_geometry(int n);
+// scratch float4 of one row of tiles; any number of rows from 1 to `tiles`
+// gives the same bits
+size_t allpairs_sym_row_f4(int n);
+int launch_allpairs_sym(int n, const float4* pos, float4* acc, float4* vel, float eps2,
+                        float G, float half_dt, float4* scratch, size_t scratch_f4,
+                        cudaStream_t st);
+int warm_allpairs_sym_kernels();
+
 // ---------------------------------------------------------------------------
 // Tuning table (tune.cu): per device, measured on it at first use or loaded
 // from its cache file.
@@ -418,6 +441,41 @@ struct EnsArgs {
   int* walk_ctr;
 };
 
+// Arguments of the pairs-once kernel for the tiles [ta, tb) of one simulation.
+struct SymArgs {
+  const float4* __restrict__ pos;
+  float4* acc;
+  float4* vel;          // closing kick or nullptr
+  float4* row;          // [tb - ta][n] tile I's sums for later targets
+  float4* col;          // [chunks][(tb - ta) * tile] chunk c's sums for tile I
+  float eps2, G, half_dt;
+  int n;
+  int tile, chunk, tiles, chunks;
+  int ta, tb;
+};
+static_assert(sizeof(SymArgs) % 8 == 0, "tables of SymArgs are followed by 8-byte entries");
+
+// The pairs-once work of a batch: an entry per simulation and pass over its
+// rows of tiles, one CTA per item and per reduction block.
+struct SymPlan {
+  struct Pass {
+    int first_item, items, first_block, blocks, chunk;
+  };
+  std::vector<SymArgs> args;
+  std::vector<int> sim, pass;
+  std::vector<size_t> region;   // pool offset (float4)
+  std::vector<int4> items;      // (entry, tile, chunk, -)
+  std::vector<int2> blocks;     // (entry, block of targets)
+  std::vector<Pass> passes;
+  unsigned char* d_table = nullptr;   // bytes(), owned by the batch
+  void clear();
+  void add(int s, const SimDesc& d, size_t at, size_t region_f4);
+  void finish();
+  size_t bytes() const;
+  int bind(const SimDesc* sims, const EnsArgs& e, float4* pool, cudaStream_t st);
+  int launch(const EnsArgs& e, cudaStream_t st) const;
+};
+
 // All-pairs work of the simulations of a batch that use the all-pairs
 // module (k_allpairs.cu): each has a region of a float4 pool holding its
 // packed sources, its partials and its tile tickets, its own launch geometry
@@ -433,7 +491,8 @@ struct EnsAllPairs {
   std::vector<int4> items;     // (all-pairs simulation, target tile, chunk, -)
   std::vector<Group> groups;
   std::vector<int> src_off;    // per simulation: pool offset of its packed
-                               // sources, -1 for one without all-pairs work
+                               // sources, -1 for one without any
+  SymPlan sym;                 // the simulations of the pairs-once kernel
   // device (owned by the batch)
   float4* d_pool = nullptr;
   APArgs* d_args = nullptr;
@@ -442,11 +501,15 @@ struct EnsAllPairs {
   int* d_counter = nullptr;    // [6] one per launch shape
 };
 // Pool float4 of one simulation's region (sources, partials, tickets); its
-// sources come first and must start zeroed, its tickets too.
+// sources come first and must start zeroed, its tickets too.  A simulation of
+// the pairs-once kernel keeps its table of partials there, whole with
+// ap_region_whole_f4, in passes over as many rows as fit with less.
 size_t ap_region_f4(int n);
+size_t ap_region_whole_f4(int n);
 // Host plan of the simulations whose SimDesc.force is NB_FORCE_NAIVE and that
 // are active: geometry, items, and the region of simulation s at
-// region_of[s] (nullptr: back to back from 0).  With region_cap, a simulation
+// region_of[s] (nullptr: back to back from 0, whole tables while they sum up to
+// 1 GiB at most).  With region_cap, a simulation
 // whose geometry now needs more than region_cap[s] float4 (the tuning table
 // changed since its region was sized) is left out and counted in *too_small.
 // Returns the pool size used.

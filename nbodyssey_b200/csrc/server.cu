@@ -100,6 +100,7 @@ struct nb_server {
   std::vector<size_t> ap_region_cap; // by sim id: region size (float4)
   EnsAllPairs ap;
   size_t ap_items_cap = 0;
+  size_t ap_sym_cap = 0;             // bytes of the pairs-once table
   bool any_tree = false;
   std::vector<int> walk_items[2];    // the walk queue (host copy)
   int* d_walk_items[2] = {nullptr, nullptr};
@@ -184,6 +185,14 @@ void give_range(std::map<int, int>& fl, int start, int len) {
 }
 
 int ap_chunks_of(int n) { return (int)((ap_region_f4(n) + kApChunk - 1) / kApChunk); }
+
+// The region a request takes: its whole table of partials when that is at most
+// 1/64 of the pool (as many requests run side by side as before), else the
+// least it can run with.
+int ap_chunks_taken(const nb_server* s, int n) {
+  const size_t whole = (ap_region_whole_f4(n) + kApChunk - 1) / kApChunk;
+  return whole * 64 <= (size_t)s->ap_chunks ? (int)whole : ap_chunks_of(n);
+}
 
 int mkdirs(const std::string& path) {
   std::string cur;
@@ -270,18 +279,18 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
     if (s->free_ids.empty()) break;
     int ap0 = -1;
     if (r->force == NB_FORCE_NAIVE) {
-      ap0 = take_range(s->ap_free, ap_chunks_of(r->n));
+      ap0 = take_range(s->ap_free, ap_chunks_taken(s, r->n));
       if (ap0 < 0) { ++k; continue; }
     }
     const int b0 = take_range(s->free_blocks, nb32);
     if (b0 < 0) {
-      if (ap0 >= 0) give_range(s->ap_free, ap0, ap_chunks_of(r->n));
+      if (ap0 >= 0) give_range(s->ap_free, ap0, ap_chunks_taken(s, r->n));
       ++k;
       continue;
     }
     if (ap0 >= 0) {
       r->ap_chunk = ap0;
-      r->ap_len = ap_chunks_of(r->n);
+      r->ap_len = ap_chunks_taken(s, r->n);
       // sources start with zero-mass pads and tickets at zero
       NB_CUDA(cudaMemsetAsync(s->d_ap_pool + (size_t)ap0 * kApChunk, 0,
                               sizeof(float4) * kApChunk * (size_t)r->ap_len, s->stream));
@@ -365,6 +374,15 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
       const size_t cap = std::max(s->ap.items.size() * 2, (size_t)4096);
       NB_CUDA(cudaMalloc(&s->ap.d_items, sizeof(int4) * cap));
       s->ap_items_cap = cap;
+    }
+    if (s->ap.sym.bytes() > s->ap_sym_cap) {   // grow-only, rare
+      NB_CUDA(cudaStreamSynchronize(s->stream));
+      if (s->ap.sym.d_table) cudaFree(s->ap.sym.d_table);
+      s->ap.sym.d_table = nullptr;
+      s->ap_sym_cap = 0;
+      const size_t cap = std::max(s->ap.sym.bytes() * 2, (size_t)1 << 16);
+      NB_CUDA(cudaMalloc((void**)&s->ap.sym.d_table, cap));
+      s->ap_sym_cap = cap;
     }
     NB_TRY(bind_ens_allpairs(s->ap, s->sims.data(), nsims, s->e, s->stream));
     plan_walk_queue(s->sims.data(), nsims, s->walk_items);
@@ -623,6 +641,7 @@ int nb_server_destroy(nb_server* s) {
   }
   for (void* p : s->dallocs) cudaFree(p);
   if (s->ap.d_items) cudaFree(s->ap.d_items);
+  if (s->ap.sym.d_table) cudaFree(s->ap.sym.d_table);
   if (s->h_frame) cudaFreeHost(s->h_frame);
   cudaStreamDestroy(s->stream);
   cudaStreamDestroy(s->side);
