@@ -12,9 +12,11 @@
 // * an internal child is accepted by every target when even the nearest point
 //   of the box of the 32 targets accepts it (size2 < theta2 * dmin2 with a
 //   1e-5 relative margin, far above the few-ulp rounding of the exact test);
-// * warp semantics: otherwise the group's extreme target along the child's
-//   dominant direction is tested exactly, and its rejection opens the child
-//   (a farthest-box-point rejection implies it, so that test is not needed);
+// * warp semantics: otherwise the group's target furthest out in the direction
+//   of the child's octant (seen from the box centre) is tested exactly, and its
+//   rejection opens the child; it settles 961 of the 1,083 opened children per
+//   warp at 1M particles (the extreme along the dominant axis, 918, and takes
+//   twice the instructions to pick);
 // * thread semantics: a child that even the farthest box point rejects is
 //   rejected by every target;
 // * the children still undecided are staged in shared memory and every lane
@@ -29,11 +31,17 @@
 // accept a child take it (an entry with their mask) and the others pass it on
 // opened.  Either way every target gets exactly the reference's set.
 //
-// Entries go to a 128-entry ring per warp (pairs interleaved as
-// (x0,x1,y0,y1)(z0,z1,m0,m1)), evaluated 32 at a time by an unrolled body
+// Entries go to a 128-entry ring per warp (planes of x, y, z and m, so that
+// the lanes' stores fall in different banks and one 16-byte load gives a
+// coordinate of two packed pairs), evaluated 32 at a time by an unrolled body
 // with packed FP32 math, two entries per instruction; entries whose mask
 // excludes a lane contribute with mass 0.  A stack that would overflow hands
 // the warp to a depth-first walk of the same semantics over the same records.
+//
+// Bound: issue slots (76 % busy) and the shared-memory pipe (77 %) together,
+// the FMA pipe 52 %: 0.95 ms and 773M warp instructions at 1M particles, theta
+// 0.5, warp semantics (0.998 ms and 811M with dominant-axis extremes, a 64-bit
+// vote mask and pair-interleaved entries).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -54,21 +62,17 @@ struct PairSmem {
   int stk[W][kPStack];
   unsigned smask[W][MASKED ? kPStack : 1];
   __align__(16) float ent[W][kPRing * 4];
-  unsigned emask[W][MASKED ? kPRing : 1];
+  __align__(16) unsigned emask[W][MASKED ? kPRing : 4];
   __align__(16) float amb[W][kPAmb * 4];
   unsigned res[W][kPAmb];
-  float4 ext[W][MASKED ? 1 : 6];
+  float4 ext[W][MASKED ? 1 : 8];
 };
 
 __device__ __forceinline__ float pw_min(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  return ord2f(__reduce_min_sync(0xffffffffu, f2ord(v)));
 }
 __device__ __forceinline__ float pw_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  return ord2f(__reduce_max_sync(0xffffffffu, f2ord(v)));
 }
 
 // (v, v) in one register pair, made at each use (volatile: not hoisted and
@@ -82,12 +86,11 @@ __device__ __forceinline__ f2 pk2u(float v) {
 // Writes one list entry (x, y, z, m) at ring position k.
 __device__ __forceinline__ void put_entry(float* ent, int k, float x, float y,
                                           float z, float m) {
-  k &= kPRing - 1;
-  float* p = &ent[(k >> 1) * 8 + (k & 1)];
+  float* p = &ent[k & (kPRing - 1)];
   p[0] = x;
-  p[2] = y;
-  p[4] = z;
-  p[6] = m;
+  p[kPRing] = y;
+  p[2 * kPRing] = z;
+  p[3 * kPRing] = m;
 }
 
 // Squared distance from (cx, cy, cz) to the nearest / farthest point of the
@@ -239,22 +242,21 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
   const float4 bi = a.ps[live ? t : n - 1];
   const float lox = pw_min(bi.x), loy = pw_min(bi.y), loz = pw_min(bi.z);
   const float hix = pw_max(bi.x), hiy = pw_max(bi.y), hiz = pw_max(bi.z);
+  const float cmx = 0.5f * (lox + hix), cmy = 0.5f * (loy + hiy), cmz = 0.5f * (loz + hiz);
   const float theta2 = a.theta2;
   const float th_lo = theta2 * 0.99999f, th_hi = theta2 * 1.00001f;
   if (!MASKED) {
-    // the targets at the group's extremes (warp semantics: one rejecting
-    // target opens a child for all)
-    const float lv[6] = {lox, hix, loy, hiy, loz, hiz};
+    // the target furthest out in each octant's direction (warp semantics: one
+    // rejecting target opens a child for all); any live target serves, so the
+    // score's low bits give way to the lane
+    const float ux = bi.x - cmx, uy = bi.y - cmy, uz = bi.z - cmz;
 #pragma unroll
-    for (int e = 0; e < 6; ++e) {
-      const float c = (e < 2) ? bi.x : (e < 4 ? bi.y : bi.z);
-      const int src = __ffs(__ballot_sync(full, c == lv[e])) - 1;
-      const float ex = __shfl_sync(full, bi.x, src), ey = __shfl_sync(full, bi.y, src),
-                  ez = __shfl_sync(full, bi.z, src);
-      if (lane == 0) sm.ext[w][e] = make_float4(ex, ey, ez, 0.f);
+    for (int o = 0; o < 8; ++o) {
+      const float score = (o & 1 ? ux : -ux) + (o & 2 ? uy : -uy) + (o & 4 ? uz : -uz);
+      const int key = (f2ord(score) & ~31) | lane;
+      if (key == __reduce_max_sync(full, key)) sm.ext[w][o] = bi;
     }
   }
-  const float cmx = 0.5f * (lox + hix), cmy = 0.5f * (loy + hiy), cmz = 0.5f * (loz + hiz);
 
   const float mx = -bi.x, my = -bi.y, mz = -bi.z;   // this lane's target, negated
   const f2 hx = pk2(mx, mx), hy = pk2(my, my), hz = pk2(mz, mz), he2 = pk2(a.eps2, a.eps2);
@@ -267,27 +269,21 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
   int head = 0;   // ring position of the first unevaluated entry (multiple of 32)
   int lc = 0;     // unevaluated entries
 
-  // list pair q of the 32-entry block at ring position `at`; (qx, qy, qz)
-  // the packed negated target and e2 the packed eps^2, made once per block
-  auto pair_term = [&](int at, int q, f2 qx, f2 qy, f2 qz, f2 e2) {
-    const float* base = &ent[at * 4];
-    const ulonglong2 A = *reinterpret_cast<const ulonglong2*>(&base[q * 8]);
-    const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(&base[q * 8 + 4]);
-    f2 m = B.y;
-    if (MASKED) {
-      // the pair's two lane masks in one load (at + 2q is even, the row
-      // 16-byte aligned); this lane's bit keeps or zeroes each mass
-      const uint2 mk = *reinterpret_cast<const uint2*>(&sm.emask[w][at + 2 * q]);
+  // a pair of list entries (masses m, lane masks m0 and m1); (qx, qy, qz) the
+  // packed negated target and e2 the packed eps^2, made once per block
+  auto pair_term = [&](f2 X, f2 Y, f2 Z, f2 m, unsigned m0, unsigned m1, f2 qx, f2 qy,
+                       f2 qz, f2 e2) {
+    if (MASKED) {   // this lane's bit keeps or zeroes each mass
       const unsigned lbit = lt + 1u;
-      const bool b0 = (mk.x & lbit) != 0u, b1 = (mk.y & lbit) != 0u;
-      float m0, m1;
-      up2(B.y, m0, m1);
-      m = pk2(b0 ? m0 : 0.f, b1 ? m1 : 0.f);
+      const bool b0 = (m0 & lbit) != 0u, b1 = (m1 & lbit) != 0u;
+      float w0, w1;
+      up2(m, w0, w1);
+      m = pk2(b0 ? w0 : 0.f, b1 ? w1 : 0.f);
       if (COUNT) cnt += (int)b0 + (int)b1;
     }
-    f2 dx = add2(A.x, qx);
-    f2 dy = add2(A.y, qy);
-    f2 dz = add2(B.x, qz);
+    f2 dx = add2(X, qx);
+    f2 dy = add2(Y, qy);
+    f2 dz = add2(Z, qz);
     f2 r2 = fma2(dz, dz, e2);
     r2 = fma2(dy, dy, r2);
     r2 = fma2(dx, dx, r2);
@@ -301,11 +297,24 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
     ay = fma2(dy, f, ay);
     az = fma2(dz, f, az);
   };
+  // list entries 4q .. 4q + 3 of the block at ring position `at` (the second
+  // pair only when asked)
+  auto quad_term = [&](int at, int q, bool second, f2 qx, f2 qy, f2 qz, f2 e2) {
+    const float* base = &ent[at + 4 * q];
+    const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(base);
+    const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(base + kPRing);
+    const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(base + 2 * kPRing);
+    const ulonglong2 M = *reinterpret_cast<const ulonglong2*>(base + 3 * kPRing);
+    uint4 mk = make_uint4(0u, 0u, 0u, 0u);
+    if (MASKED) mk = *reinterpret_cast<const uint4*>(&sm.emask[w][at + 4 * q]);
+    pair_term(X.x, Y.x, Z.x, M.x, mk.x, mk.y, qx, qy, qz, e2);
+    if (second) pair_term(X.y, Y.y, Z.y, M.y, mk.z, mk.w, qx, qy, qz, e2);
+  };
   // evaluates the 32 entries at `head` (unrolled, fixed offsets)
   auto flush_full = [&]() {
     const f2 qx = px(), qy = py(), qz = pz(), e2 = HOIST ? he2 : pk2u(a.eps2);
 #pragma unroll
-    for (int q = 0; q < kPFlush / 2; ++q) pair_term(head, q, qx, qy, qz, e2);
+    for (int q = 0; q < kPFlush / 4; ++q) quad_term(head, q, true, qx, qy, qz, e2);
     if (!MASKED && COUNT) cnt += kPFlush;
     head = (head + kPFlush) & (kPRing - 1);
     lc -= kPFlush;
@@ -381,14 +390,11 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
       amb0 = has && !bacc0 && !brej0;
       amb1 = has && !bacc1 && !brej1;
     } else {
-      // the group's extreme target along the child's dominant direction
-      // from the box centre; its exact rejection opens the child
+      // the group's target furthest out in the direction of the child's
+      // octant around the box centre; its exact rejection opens the child
       auto ext_accepts = [&](float s2, float cx, float cy, float cz) {
-        const float rx = cx - cmx, ry = cy - cmy, rz = cz - cmz;
-        const float qx = fabsf(rx), qy = fabsf(ry), qz = fabsf(rz);
-        const int e = (qx >= qy && qx >= qz) ? (rx > 0.f ? 1 : 0)
-                                             : (qy >= qz ? (ry > 0.f ? 3 : 2) : (rz > 0.f ? 5 : 4));
-        const float4 q = sm.ext[w][e];
+        const int o = (cx > cmx ? 1 : 0) | (cy > cmy ? 2 : 0) | (cz > cmz ? 4 : 0);
+        const float4 q = sm.ext[w][o];
         return accepts(s2, theta2, cx, cy, cz, q.x, q.y, q.z);
       };
       amb0 = has && !bacc0 && ext_accepts(s0, c0.x, c0.y, c0.z);
@@ -422,7 +428,7 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
       // warp semantics need only "every target accepts": a vote every lane
       // receives, kept in a warp-uniform bit mask; thread semantics need the
       // accepting lanes, one ballot per child through shared memory
-      unsigned long long allacc = 0ull;
+      unsigned all0 = 0u, all1 = 0u, bit = 1u;   // bit q: pair q's first / second child
       for (int q = 0; q < (na + 1) >> 1; ++q) {
         const ulonglong2 U = *reinterpret_cast<const ulonglong2*>(&am[q * 8]);
         const ulonglong2 V = *reinterpret_cast<const ulonglong2*>(&am[q * 8 + 4]);
@@ -440,9 +446,9 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
           }
         } else {
           // a dead lane tests a copy of live target n-1
-          const unsigned long long b0 = __all_sync(full, z0 < t0) ? 1ull : 0ull;
-          const unsigned long long b1 = __all_sync(full, z1 < t1) ? 2ull : 0ull;
-          allacc |= (b0 | b1) << (2 * q);
+          if (__all_sync(full, z0 < t0)) all0 |= bit;
+          if (__all_sync(full, z1 < t1)) all1 |= bit;
+          bit += bit;
         }
       }
       if (MASKED) {
@@ -450,8 +456,8 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
         if (amb0) r0 = sm.res[w][ka0];
         if (amb1) r1 = sm.res[w][ka1];
       } else {
-        r0 = (unsigned)(allacc >> ka0) & 1u;
-        r1 = (unsigned)(allacc >> ka1) & 1u;
+        r0 = ((ka0 & 1 ? all1 : all0) >> (ka0 >> 1)) & 1u;
+        r1 = ((ka1 & 1 ? all1 : all0) >> (ka1 >> 1)) & 1u;
       }
     }
     // accepting targets of each child
@@ -508,7 +514,7 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
       }
       const int np = (lc + 1) >> 1;
       const f2 qx = px(), qy = py(), qz = pz(), e2 = HOIST ? he2 : pk2u(a.eps2);
-      for (int q = 0; q < np; ++q) pair_term(head, q, qx, qy, qz, e2);
+      for (int q = 0; q < np; q += 2) quad_term(head, q >> 1, q + 1 < np, qx, qy, qz, e2);
       if (!MASKED && COUNT) cnt += lc;
     }
     float u, v;
@@ -531,13 +537,15 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
   }
 }
 
-// At most 64 registers a thread: 32 warps resident per SM whatever the block
-// shape (the compiler otherwise takes 70 for 8-warp blocks).
+// Warp semantics: at most 64 registers a thread, 32 warps resident per SM
+// whatever the block shape (the compiler otherwise takes 70 for 8-warp blocks).
+// Thread semantics: 72, 28 warps, which keep the packed target live through
+// the walk (1.51 ms at 1M against 1.55 with 64 registers, 1.53 with 80).
 template <int W, bool MASKED, bool COUNT>
-__global__ void __launch_bounds__(W * 32, 32 / W) k_walk_pair(WalkArgs a) {
+__global__ void __launch_bounds__(W * 32, (MASKED ? 28 : 32) / W) k_walk_pair(WalkArgs a) {
   __shared__ PairSmem<W, MASKED> sm;
   chain_wait();
-  walk_pair_warp<W, MASKED, COUNT>(a, a.t0 / 32 + blockIdx.x * W + (threadIdx.x >> 5), sm);
+  walk_pair_warp<W, MASKED, COUNT, MASKED>(a, a.t0 / 32 + blockIdx.x * W + (threadIdx.x >> 5), sm);
 }
 
 
@@ -546,9 +554,13 @@ __global__ void __launch_bounds__(W * 32, 32 / W) k_walk_pair(WalkArgs a) {
 // (costliest simulations first, so the longest walks do not start last) and
 // walk each with that block's simulation: its tree, parameters and
 // semantics.  Blocks belong to one simulation (bases are multiples of 32).
+//
+// Registers: 64 a thread for warp semantics (at 72 with the packed target kept
+// live the compiler spills 1 KB: 355 us a step of 24 encounters against 353),
+// 80 for thread semantics with it kept live (463 us against 481 at 64).
 constexpr int kEnsW = 4;
 template <bool MASKED>
-__global__ void __launch_bounds__(kEnsW * 32) k_walk_pair_ens(EnsArgs e) {
+__global__ void __launch_bounds__(kEnsW * 32, MASKED ? 6 : 8) k_walk_pair_ens(EnsArgs e) {
   __shared__ PairSmem<kEnsW, MASKED> sm;
   const int lane = threadIdx.x & 31;
   const int* items = e.walk_items[MASKED ? 1 : 0];
@@ -587,7 +599,7 @@ __global__ void __launch_bounds__(kEnsW * 32) k_walk_pair_ens(EnsArgs e) {
     a.t0 = 0;
     a.t1 = d.n;
     a.part = nullptr;
-    walk_pair_warp<kEnsW, MASKED, false, true>(a, blk - d.base / 32, sm);
+    walk_pair_warp<kEnsW, MASKED, false, MASKED>(a, blk - d.base / 32, sm);
     __syncwarp();   // this warp's shared memory is free for its next block
   }
 }
