@@ -336,9 +336,15 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   NB_TRY(launch_prep(w, a, true, false, st));
   if (a.after_prep) NB_CUDA(cudaEventRecord(a.after_prep, st));
   NB_TRY(mark(pm, NB_PHASE_PREP, st));
-  NB_TRY(launch_morton(w, a, st));
-  NB_TRY(mark(pm, NB_PHASE_MORTON, st));
-  NB_TRY(launch_sort(w, a, st));
+  if (sort_in_cluster(a.n, a.key_bits)) {
+    // the keys are made in the sort's launch: their phase is the event's own
+    NB_TRY(mark(pm, NB_PHASE_MORTON, st));
+    NB_TRY(launch_sort_cluster(w, a, st));
+  } else {
+    NB_TRY(launch_morton(w, a, st));
+    NB_TRY(mark(pm, NB_PHASE_MORTON, st));
+    NB_TRY(launch_sort(w, a, st));
+  }
   NB_TRY(mark(pm, NB_PHASE_SORT, st));
   NB_TRY(launch_build(w, a, st));
   NB_TRY(mark(pm, NB_PHASE_BUILD, st));

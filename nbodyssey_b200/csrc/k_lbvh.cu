@@ -4,9 +4,15 @@
 //   Karras radix tree + bottom-up centres of mass / boxes / sizes (FP64
 //   mass-weighted sums): one fused bottom-up build in levels, for a single
 //   tree or for all the trees of an ensemble at once.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cuda/atomic>
+#include <mutex>
 
 #include "nb_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace nb {
 
@@ -40,6 +46,19 @@ __device__ __forceinline__ uint32_t quantise(float p, float lo, float inv,
   return (uint32_t)fminf(__fmul_rn(fmaxf(t, 0.f), scale), qmax);
 }
 
+// Morton key of a particle in the box [lx, lx + 1 / inv] x ... (10 or 21 bits
+// per axis by the key type).
+template <typename K>
+__device__ __forceinline__ K morton_key(float4 p, float lx, float ly, float lz, float inv) {
+  constexpr bool wide = sizeof(K) == 8;
+  constexpr float scale = wide ? 2097152.f : 1024.f;
+  const uint32_t qx = quantise(p.x, lx, inv, scale, scale - 1.f);
+  const uint32_t qy = quantise(p.y, ly, inv, scale, scale - 1.f);
+  const uint32_t qz = quantise(p.z, lz, inv, scale, scale - 1.f);
+  if (wide) return (K)((spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz));
+  return (K)((spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz));
+}
+
 constexpr int kMortonThreads = 1024;
 
 template <typename K>
@@ -56,9 +75,6 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const float4* __restr
   const float ext =
       fmaxf(__fsub_rn(hx, lx), fmaxf(__fsub_rn(hy, ly), __fsub_rn(hz, lz)));
   const float inv = ext > 0.f ? __frcp_rn(ext) : 0.f;
-  const bool wide = sizeof(K) == 8;
-  const float scale = wide ? 2097152.f : 1024.f;
-  const float qmax = scale - 1.f;
   // four particles per thread and round, their loads issued together
   const int stride = gridDim.x * blockDim.x;
   for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
@@ -72,15 +88,7 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const float4* __restr
     for (int u = 0; u < 4; ++u) {
       const int i = i0 + u * stride;
       if (i >= n) break;
-      const float4 p = pv[u];
-      uint32_t qx = quantise(p.x, lx, inv, scale, qmax);
-      uint32_t qy = quantise(p.y, ly, inv, scale, qmax);
-      uint32_t qz = quantise(p.z, lz, inv, scale, qmax);
-      K k;
-      if (wide)
-        k = (K)((spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz));
-      else
-        k = (K)((spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz));
+      const K k = morton_key<K>(pv[u], lx, ly, lz, inv);
       keys[i] = k;
       for (int ps = 0; ps < passes; ++ps)
         atomicAdd(&s_hist[ps * kSortRadix + (uint32_t)((k >> (8 * ps)) & 0xffu)], 1u);
@@ -418,6 +426,298 @@ static int sort_impl(Workspace& w, const StepArgs& a, cudaStream_t st) {
 int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st) {
   if (a.key_bits == 63) return sort_impl<uint64_t>(w, a, st);
   return sort_impl<uint32_t>(w, a, st);
+}
+
+// ---------------------------------------------------------------------------
+// Morton keys and the whole sort in one launch, for n up to kClusterMax: a
+// cluster of 16 CTAs holds all keys and values in its shared memory, ranks its
+// slice of them each pass as the onesweep kernel does, sends its digit counts
+// to the others over distributed shared memory in place of the look-back, and
+// writes each digit's run into the slices it belongs to; the last pass writes
+// the keys, the permutation and the gathered positions to global memory.  The
+// same stable sort, so the same permutation.
+//
+// Bound: latency.  Up to about 100,000 keys a onesweep pass takes 9 us whatever
+// n is (launch, ticket, look-back); here a pass is two cluster barriers (0.5 us
+// each), and the rank (0.5 us for every 1,024 keys of a slice) and scatter of
+// n / 16 keys per SM: 20 us for the keys and four passes at n = 4,096 against
+// 42, 27 against 47 at 20,011, 45 against 51 at 65,536.  512 threads: with 1,024
+// the barriers cost more than the wider rank gains (31 us at 20,011).
+// ---------------------------------------------------------------------------
+constexpr int kClusterCtas = 16;
+constexpr int kClusterThreads = 512;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterParts = kClusterThreads / kSortRadix;   // eight warps each
+constexpr int kClusterItems = 8;
+constexpr int kClusterSlice = kClusterThreads * kClusterItems;   // keys per CTA at most
+constexpr int kClusterMax = kClusterCtas * kClusterSlice;
+
+__host__ __device__ constexpr size_t cluster_sort_smem(size_t key_bytes, int slice) {
+  // keys and values twice, digit counts by warp, by part of the warps and by
+  // CTA (twice), two words per digit, and scan words
+  return 2 * (size_t)slice * (key_bytes + 4) + kClusterWarps * kSortRadix * 2 +
+         kClusterParts * kSortRadix * 4 + (2 * kClusterCtas + 2) * kSortRadix * 4 + 16 * 4;
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    k_sort_cluster(const float4* __restrict__ pos, int n, const int* __restrict__ bbox,
+                   K* __restrict__ kout, uint32_t* __restrict__ vout,
+                   float4* __restrict__ pos_sorted, int slice, uint32_t slice_inv, int passes,
+                   unsigned* err) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  K* s_key = reinterpret_cast<K*>(s_raw);                               // [2][slice]
+  uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + 2 * slice);     // [2][slice]
+  uint16_t* s_wc = reinterpret_cast<uint16_t*>(s_val + 2 * slice);      // [warps][radix]
+  uint32_t* s_part = reinterpret_cast<uint32_t*>(s_wc + kClusterWarps * kSortRadix);   // [parts][radix]
+  uint32_t* s_cnt = s_part + kClusterParts * kSortRadix;     // [2][CTAs][radix] digit counts
+  uint32_t* s_tex = s_cnt + 2 * kClusterCtas * kSortRadix;      // digit's first place in the slice
+  uint32_t* s_base = s_tex + kSortRadix;         // slice place -> global place
+  uint32_t* s_scan = s_base + kSortRadix;        // [2][8]
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cta = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const int first = cta * slice;
+  const int count = max(0, min(slice, n - first));
+  const int items = (slice + kClusterThreads - 1) / kClusterThreads;
+  const int seg = warp * items * 32 + lane;
+  cluster.barrier_arrive();   // waited for before the first remote store: every CTA has started
+  chain_release();
+  chain_wait();
+
+  K key[kClusterItems];
+  uint32_t val[kClusterItems];
+  {
+    const float lx = ord2f(bbox[0]), ly = ord2f(bbox[1]), lz = ord2f(bbox[2]);
+    const float hx = ord2f(bbox[3]), hy = ord2f(bbox[4]), hz = ord2f(bbox[5]);
+    const float ext =
+        fmaxf(__fsub_rn(hx, lx), fmaxf(__fsub_rn(hy, ly), __fsub_rn(hz, lz)));
+    const float inv = ext > 0.f ? __frcp_rn(ext) : 0.f;
+#pragma unroll
+    for (int k = 0; k < kClusterItems; ++k) {
+      const int i = seg + 32 * k;
+      if (k < items && i < count) {
+        key[k] = morton_key<K>(pos[first + i], lx, ly, lz, inv);
+        val[k] = (uint32_t)(first + i);
+      }
+    }
+  }
+  for (int ps = 0; ps < passes; ++ps) {
+    const int shift = 8 * ps;
+    K* ck = s_key + (ps & 1) * slice;             // this pass's slice, then its staging
+    uint32_t* cv = s_val + (ps & 1) * slice;
+    K* nk = s_key + ((ps + 1) & 1) * slice;       // the next pass's slice
+    uint32_t* nv = s_val + ((ps + 1) & 1) * slice;
+    uint32_t* cnt = s_cnt + (ps & 1) * kClusterCtas * kSortRadix;
+    reinterpret_cast<uint4*>(s_wc)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    if (ps > 0) {
+#pragma unroll
+      for (int k = 0; k < kClusterItems; ++k) {
+        const int i = seg + 32 * k;
+        if (k < items && i < count) {
+          key[k] = ck[i];
+          val[k] = cv[i];
+        }
+      }
+    }
+    __syncthreads();
+    uint32_t rank[kClusterItems];
+    uint16_t* wc = s_wc + warp * kSortRadix;
+#pragma unroll
+    for (int k = 0; k < kClusterItems; ++k) {
+      if (k >= items) break;
+      const bool ok = seg + 32 * k < count;
+      const uint32_t d = ok ? (uint32_t)((key[k] >> shift) & 0xffu) : 0u;
+      const uint32_t peers = digit_peers(d, ok);
+      uint32_t old = 0;
+      if (ok) {
+        old = wc[d];
+        rank[k] = old + __popc(peers & lt);
+      }
+      __syncwarp();
+      if (ok && lane == __ffs(peers) - 1) wc[d] = (uint16_t)(old + __popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    // thread (q, d): the counts of digit d in eight warps
+    const int d = tid & (kSortRadix - 1), q = tid >> 8;
+    uint32_t run = 0;
+    uint16_t* col = s_wc + q * 8 * kSortRadix + d;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) run += col[w * kSortRadix];
+    s_part[q * kSortRadix + d] = run;
+    __syncthreads();
+    uint32_t before = 0, mine = 0;
+#pragma unroll
+    for (int p = 0; p < kClusterParts; ++p) {
+      const uint32_t c = s_part[p * kSortRadix + d];
+      before += p < q ? c : 0u;
+      mine += c;
+    }
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {   // exclusive over the warps
+      const uint32_t c = col[w * kSortRadix];
+      col[w * kSortRadix] = (uint16_t)before;
+      before += c;
+    }
+    if (ps == 0) cluster.barrier_wait();
+    // this CTA's counts to every CTA (stored there: a load from another SM's
+    // shared memory would wait its whole latency)
+#pragma unroll
+    for (int r = q; r < kClusterCtas; r += kClusterParts)
+      cluster.map_shared_rank(cnt, r)[cta * kSortRadix + d] = mine;
+    cluster.sync();
+    // digit threads: this CTA's counts and all CTAs' counts, scanned by digit
+    uint32_t lower = 0, total = 0, tin = 0, gin = 0;
+    if (q == 0) {
+#pragma unroll
+      for (int r = 0; r < kClusterCtas; ++r) {
+        const uint32_t c = cnt[r * kSortRadix + d];
+        lower += r < cta ? c : 0u;
+        total += c;
+      }
+      tin = mine;
+      gin = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, tin, o);
+        const uint32_t y = __shfl_up_sync(0xffffffffu, gin, o);
+        if (lane >= o) {
+          tin += x;
+          gin += y;
+        }
+      }
+      if (lane == 31) {
+        s_scan[warp] = tin;
+        s_scan[8 + warp] = gin;
+      }
+    }
+    __syncthreads();
+    if (q == 0) {
+      uint32_t tofs = 0, gofs = 0;
+      for (int i = 0; i < warp; ++i) {
+        tofs += s_scan[i];
+        gofs += s_scan[8 + i];
+      }
+      const uint32_t tex = tofs + tin - mine;
+      s_tex[d] = tex;
+      s_base[d] = gofs + gin - total + lower - tex;   // unsigned wrap-around cancels
+    }
+    __syncthreads();
+    // the slice in digit order, over the pass's own keys (all in registers)
+#pragma unroll
+    for (int k = 0; k < kClusterItems; ++k) {
+      if (k < items && seg + 32 * k < count) {
+        const uint32_t dg = (uint32_t)((key[k] >> shift) & 0xffu);
+        const uint32_t at = s_tex[dg] + wc[dg] + rank[k];
+        if (at < (uint32_t)count) {
+          ck[at] = key[k];
+          cv[at] = val[k];
+        } else {
+          raise_err(err, NB_DEVERR_SORT);
+        }
+      }
+    }
+    __syncthreads();
+    const bool last = ps == passes - 1;
+#pragma unroll
+    for (int k = 0; k < kClusterItems; ++k) {
+      const int i = tid + k * kClusterThreads;
+      if (i >= count) break;
+      const K kk = ck[i];
+      const uint32_t vv = cv[i];
+      const uint32_t p = s_base[(uint32_t)((kk >> shift) & 0xffu)] + (uint32_t)i;
+      if (p >= (uint32_t)n || vv >= (uint32_t)n) {
+        raise_err(err, NB_DEVERR_SORT);
+        continue;
+      }
+      if (last) {
+        kout[p] = kk;
+        vout[p] = vv;
+        pos_sorted[p] = pos[vv];
+      } else {
+        const uint32_t r = __umulhi(p, slice_inv);   // p / slice
+        cluster.map_shared_rank(nk, r)[p - r * slice] = kk;
+        cluster.map_shared_rank(nv, r)[p - r * slice] = vv;
+      }
+    }
+    if (!last) cluster.sync();   // the next slice is complete
+  }
+}
+
+template <typename K>
+static int cluster_sort_config(int slice, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = kClusterCtas;
+  cfg->blockDim = kClusterThreads;
+  cfg->dynamicSmemBytes = cluster_sort_smem(sizeof(K), slice);
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClusterCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+  NB_CUDA(cudaFuncSetAttribute(k_sort_cluster<K>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                               1));
+  NB_CUDA(cudaFuncSetAttribute(k_sort_cluster<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)cluster_sort_smem(sizeof(K), kClusterSlice)));
+  return NB_OK;
+}
+
+// Whether the device can hold the cluster (16 CTAs is above the portable 8, and
+// a partitioned device may have no 16 SMs together): asked once per device.
+template <typename K>
+static bool cluster_sort_fits() {
+  static std::mutex mu;
+  static int known[64] = {};   // 0 not asked, 1 yes, 2 no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    cudaGetLastError();
+    return false;
+  }
+  std::lock_guard<std::mutex> lk(mu);
+  if (!known[dev]) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    int clusters = 0;
+    const bool ok = cluster_sort_config<K>(kClusterSlice, &cfg, at) == NB_OK &&
+                    cudaOccupancyMaxActiveClusters(&clusters, k_sort_cluster<K>, &cfg) ==
+                        cudaSuccess &&
+                    clusters >= 1;
+    if (!ok) cudaGetLastError();
+    known[dev] = ok ? 1 : 2;
+  }
+  return known[dev] == 1;
+}
+
+// Step of a simulation, one launch against Morton kernel and onesweep passes:
+// 30 bits 52 against 66 us at n = 1,000, 115 / 136 at 20,011, 161 / 164 at 65,536;
+// 63 bits 134 / 168 at 20,011, 181 / 197 at 50,000, equal near 65,536 (8 passes
+// over n / 16 keys per SM, while the onesweep's grow little with n).
+bool sort_in_cluster(int n, int key_bits) {
+  if (n > (key_bits == 63 ? kClusterMax * 3 / 4 : kClusterMax)) return false;
+  return key_bits == 63 ? cluster_sort_fits<uint64_t>() : cluster_sort_fits<uint32_t>();
+}
+
+template <typename K>
+static int cluster_sort(Workspace& w, const StepArgs& a, cudaStream_t st) {
+  // whole warps of keys; n / slice by a multiplication, exact for n < 2^17
+  const int slice = std::max(32, ((a.n + kClusterCtas - 1) / kClusterCtas + 31) / 32 * 32);
+  const uint32_t inv = (uint32_t)((((uint64_t)1 << 32) + slice - 1) / slice);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  NB_TRY(cluster_sort_config<K>(slice, &cfg, at));
+  cfg.stream = st;
+  chained_attribute(st, &cfg, at);
+  NB_CUDA(cudaLaunchKernelEx(&cfg, k_sort_cluster<K>, (const float4*)a.pos, a.n,
+                             (const int*)w.bbox, (K*)w.keys, w.vals, w.pos_sorted, slice, inv,
+                             sort_passes(a.key_bits), w.err));
+  return NB_OK;
+}
+
+int launch_sort_cluster(Workspace& w, const StepArgs& a, cudaStream_t st) {
+  if (a.key_bits == 63) return cluster_sort<uint64_t>(w, a, st);
+  return cluster_sort<uint32_t>(w, a, st);
 }
 
 __device__ __forceinline__ int clz_k(uint32_t x) { return __clz((int)x); }
@@ -1218,6 +1518,7 @@ int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st) 
 
 int warm_lbvh_kernels() {
   return warm_fns(k_morton<uint32_t>, k_morton<uint64_t>, k_ens_morton,
+                  k_sort_cluster<uint32_t>, k_sort_cluster<uint64_t>,
                   k_sort_pass<uint32_t, kSortMid>, k_sort_pass<uint32_t, kSortLast>,
                   k_sort_pass<uint64_t, kSortMid>, k_sort_pass<uint64_t, kSortLast>,
                   k_sort_pass<uint64_t, kSortLastEnsemble>, k_build_level<uint32_t, true>,

@@ -180,6 +180,10 @@ int launch_prep(Workspace& w, const StepArgs& a, bool bbox, bool pack,
                 cudaStream_t st);
 int launch_morton(Workspace& w, const StepArgs& a, cudaStream_t st);
 int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st);
+// Morton keys and sort in one launch, for sizes that fit a cluster's shared
+// memory (on a device that can hold it); the sort scratch is not used
+bool sort_in_cluster(int n, int key_bits);
+int launch_sort_cluster(Workspace& w, const StepArgs& a, cudaStream_t st);
 size_t build_seg_entries(int cap);
 int launch_build(Workspace& w, const StepArgs& a, cudaStream_t st);
 int launch_com(Workspace& w, const StepArgs& a, cudaStream_t st);
@@ -244,6 +248,19 @@ __device__ __forceinline__ void chain_wait() {
 __device__ __forceinline__ void chain_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Adds the attribute to a launch of the chain (room for one more in `at`).
+inline void chained_attribute(cudaStream_t st, cudaLaunchConfig_t* cfg,
+                              cudaLaunchAttribute* at) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    cs = cudaStreamCaptureStatusNone;
+  }
+  if (cs != cudaStreamCaptureStatusNone) return;
+  at[cfg->numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[cfg->numAttrs].val.programmaticStreamSerializationAllowed = 1;
+  ++cfg->numAttrs;
+}
 template <typename... KArgs, typename... Args>
 inline int launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                           cudaStream_t st, Args&&... args) {
@@ -253,15 +270,8 @@ inline int launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
-    cudaGetLastError();
-    cs = cudaStreamCaptureStatusNone;
-  }
-  cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+  chained_attribute(st, &cfg, at);
   NB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
   return NB_OK;
 }
