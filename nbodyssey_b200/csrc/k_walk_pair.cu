@@ -38,10 +38,12 @@
 // excludes a lane contribute with mass 0.  A stack that would overflow hands
 // the warp to a depth-first walk of the same semantics over the same records.
 //
-// Bound: issue slots (76 % busy) and the shared-memory pipe (77 %) together,
-// the FMA pipe 52 %: 0.95 ms and 773M warp instructions at 1M particles, theta
-// 0.5, warp semantics (0.998 ms and 811M with dominant-axis extremes, a 64-bit
-// vote mask and pair-interleaved entries).
+// Bound: with many warps, issue slots (76 % busy) and the shared-memory pipe
+// (77 %) together, the FMA pipe 52 %: 0.94 ms and 773M warp instructions at 1M
+// particles, theta 0.5, warp semantics (0.998 ms and 811M with dominant-axis
+// extremes, a 64-bit vote mask and pair-interleaved entries).  With few, the
+// latency of a step, the record loads above all: the next step's are issued
+// before this step's entries are evaluated (20,011 particles: 57 us without).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -344,30 +346,33 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
     __syncwarp();
   }
 
-  bool overflow = false;
-  for (int guard = 0; sp > 0; ++guard) {
-    if (sp + 32 > kPStack || guard > n) {   // uniform across the warp
-      overflow = true;
-      break;
-    }
+  // takes up to 32 opened nodes off the stack, one per lane, and loads their
+  // records, on their way while the step before evaluates its entries
+  bool has = false;
+  unsigned M = live_mask;
+  float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0, sw = c0;
+  auto pop = [&]() {
     const int take = min(sp, 32);
-    const int base = sp - take;
-    const bool has = lane < take;
-    int k = 0;
-    unsigned M = live_mask;
+    sp -= take;
+    has = lane < take;
     if (has) {
-      k = sm.stk[w][base + lane];
-      if (MASKED) M = sm.smask[w][base + lane];
-    }
-    __syncwarp();
-    sp = base;
-    k = min(max(k, 0), ni - 1);   // a valid tree never needs the clamp
-    float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0, sw = c0;
-    if (has) {
+      int k = sm.stk[w][sp + lane];
+      if (MASKED) M = sm.smask[w][sp + lane];
+      k = min(max(k, 0), ni - 1);   // a valid tree never needs the clamp
       const PairRec* r = a.pairs + k;
       c0 = r->c[0];
       c1 = r->c[1];
       sw = r->sw;
+    }
+    __syncwarp();
+  };
+  bool overflow = false;
+  bool more = sp > 0;
+  if (more) pop();
+  for (int guard = 0; more; ++guard) {
+    if (sp + 64 > kPStack || guard > n) {   // uniform across the warp
+      overflow = true;
+      break;
     }
     // child j: position / centre of mass (cj.x, cj.y, cj.z), mass cj.w,
     // size2 and split in sw (.x, .y for the left child, .z, .w the right)
@@ -498,6 +503,8 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
     }
     sp += np0 + __popc(pb1);
     __syncwarp();
+    more = sp > 0;
+    if (more) pop();
     while (lc >= kPFlush) flush_full();
     __syncwarp();
   }
@@ -537,17 +544,14 @@ __device__ __forceinline__ void walk_pair_warp(const WalkArgs& a, int wg,
   }
 }
 
-// Warp semantics: at most 64 registers a thread, 32 warps resident per SM
-// whatever the block shape (the compiler otherwise takes 70 for 8-warp blocks).
-// Thread semantics: 72, 28 warps, which keep the packed target live through
-// the walk (1.51 ms at 1M against 1.55 with 64 registers, 1.53 with 80).
-template <int W, bool MASKED, bool COUNT>
-__global__ void __launch_bounds__(W * 32, (MASKED ? 28 : 32) / W) k_walk_pair(WalkArgs a) {
+// At most 65,536 / (32 x WARPS) registers a thread, so that WARPS warps are
+// resident per SM whatever the block shape.
+template <int W, int WARPS, bool MASKED, bool COUNT>
+__global__ void __launch_bounds__(W * 32, WARPS / W) k_walk_pair(WalkArgs a) {
   __shared__ PairSmem<W, MASKED> sm;
   chain_wait();
   walk_pair_warp<W, MASKED, COUNT, MASKED>(a, a.t0 / 32 + blockIdx.x * W + (threadIdx.x >> 5), sm);
 }
-
 
 // Ensembles and the server: one persistent launch per semantics.  Its warps
 // pop 32-slot blocks of the concatenated sorted arrays from a device queue
@@ -555,12 +559,11 @@ __global__ void __launch_bounds__(W * 32, (MASKED ? 28 : 32) / W) k_walk_pair(Wa
 // walk each with that block's simulation: its tree, parameters and
 // semantics.  Blocks belong to one simulation (bases are multiples of 32).
 //
-// Registers: 64 a thread for warp semantics (at 72 with the packed target kept
-// live the compiler spills 1 KB: 355 us a step of 24 encounters against 353),
-// 80 for thread semantics with it kept live (463 us against 481 at 64).
+// Registers: 80 a thread (6 blocks per SM); 24 encounters of up to 65,536
+// particles take 346 us a step with them, 350 with 72 and 352 with 64.
 constexpr int kEnsW = 4;
 template <bool MASKED>
-__global__ void __launch_bounds__(kEnsW * 32, MASKED ? 6 : 8) k_walk_pair_ens(EnsArgs e) {
+__global__ void __launch_bounds__(kEnsW * 32, 6) k_walk_pair_ens(EnsArgs e) {
   __shared__ PairSmem<kEnsW, MASKED> sm;
   const int lane = threadIdx.x & 31;
   const int* items = e.walk_items[MASKED ? 1 : 0];
@@ -637,38 +640,53 @@ int launch_walk_pair_ens(const EnsArgs& e, cudaStream_t st) {
   return NB_OK;
 }
 
-template <int W>
-static int launch_walk_pair_w(const WalkArgs& a, bool masked, int blocks, cudaStream_t st) {
-  if (masked) {
-    // the lane masks double the stack: thread semantics stay at <= 4 warps
-    // per block (<= 32 KB of static shared memory)
-    constexpr int WM = W < 4 ? W : 4;
-    const int bm = (blocks * W + WM - 1) / WM;
-    return a.counts ? launch_chained(k_walk_pair<WM, true, true>, bm, WM * 32, 0, st, a)
-                    : launch_chained(k_walk_pair<WM, true, false>, bm, WM * 32, 0, st, a);
-  }
-  return a.counts ? launch_chained(k_walk_pair<W, false, true>, blocks, W * 32, 0, st, a)
-                  : launch_chained(k_walk_pair<W, false, false>, blocks, W * 32, 0, st, a);
+template <int W, int WARPS>
+static int launch_walk_pair_w(const WalkArgs& a, bool masked, int warps, cudaStream_t st) {
+  // the lane masks double the stack: thread semantics stay at <= 4 warps per
+  // block (<= 32 KB of static shared memory)
+  constexpr int WM = W < 4 ? W : 4;
+  const int blocks = (warps + W - 1) / W, bm = (warps + WM - 1) / WM;
+  if (masked)
+    return a.counts
+               ? launch_chained(k_walk_pair<WM, WARPS, true, true>, bm, WM * 32, 0, st, a)
+               : launch_chained(k_walk_pair<WM, WARPS, true, false>, bm, WM * 32, 0, st, a);
+  return a.counts
+             ? launch_chained(k_walk_pair<W, WARPS, false, true>, blocks, W * 32, 0, st, a)
+             : launch_chained(k_walk_pair<W, WARPS, false, false>, blocks, W * 32, 0, st, a);
 }
 
-// The block shape (warps per block) is the tuning table's.
+// Warps per SM by how many there are to run: registers hide latency better
+// than warps as long as all warps are resident at once, or nearly.  Warp walk
+// with 16 / 20 / 24 warps: 45 / 47 / 51 us at 20,011 particles (4.2 warps per
+// SM), 105 / 96 / 98 at 100,000 (21), 185 / 180 / 188 at 200,000 (42), 1,003 / 950
+// / 936 at 1M (211).  With enough of them the block shape (warps per block) is
+// the tuning table's.
 int launch_walk_pair(const WalkArgs& a, bool masked, cudaStream_t st) {
   const int warps = (a.t1 - a.t0 + 31) / 32;
   if (warps <= 0) return NB_OK;
+  const int sms = device_sm_count();
+  if (warps <= 16 * sms) return launch_walk_pair_w<4, 16>(a, masked, warps, st);
+  if (warps <= 48 * sms) return launch_walk_pair_w<4, 20>(a, masked, warps, st);
   const int W = tune_walk_warps();
-  const int blocks = (warps + W - 1) / W;
-  if (W == 2) return launch_walk_pair_w<2>(a, masked, blocks, st);
-  if (W == 8) return launch_walk_pair_w<8>(a, masked, blocks, st);
-  return launch_walk_pair_w<4>(a, masked, blocks, st);
+  if (W == 2) return launch_walk_pair_w<2, 24>(a, masked, warps, st);
+  if (W == 8) return launch_walk_pair_w<8, 24>(a, masked, warps, st);
+  return launch_walk_pair_w<4, 24>(a, masked, warps, st);
+}
+
+template <int W, int WARPS>
+static int warm_walk_pair_w() {
+  constexpr int WM = W < 4 ? W : 4;
+  return warm_fns(k_walk_pair<W, WARPS, false, false>, k_walk_pair<W, WARPS, false, true>,
+                  k_walk_pair<WM, WARPS, true, false>, k_walk_pair<WM, WARPS, true, true>);
 }
 
 int warm_walk_pair_kernels() {
-  return warm_fns(k_walk_pair<2, false, false>, k_walk_pair<2, false, true>,
-                  k_walk_pair<4, false, false>, k_walk_pair<4, false, true>,
-                  k_walk_pair<8, false, false>, k_walk_pair<8, false, true>,
-                  k_walk_pair<2, true, false>, k_walk_pair<2, true, true>,
-                  k_walk_pair<4, true, false>, k_walk_pair<4, true, true>,
-                  k_walk_pair_ens<false>, k_walk_pair_ens<true>);
+  NB_TRY((warm_walk_pair_w<4, 16>()));
+  NB_TRY((warm_walk_pair_w<4, 20>()));
+  NB_TRY((warm_walk_pair_w<2, 24>()));
+  NB_TRY((warm_walk_pair_w<4, 24>()));
+  NB_TRY((warm_walk_pair_w<8, 24>()));
+  return warm_fns(k_walk_pair_ens<false>, k_walk_pair_ens<true>);
 }
 
 }  // namespace nb

@@ -266,9 +266,10 @@ int measure(nb_tune_table* t) {
     g_tab[current_device()] = *t;
   };
   install();
-  // the walk's warps per block, on the largest crossover size
+  // the walk's warps per block, at a size that launches the shapes it chooses
+  // between (more than 48 warps per SM)
   {
-    const int n = 131072;
+    const int n = 262144;
     NB_TRY(b.load(n));
     double best = 1e30;
     int best_w = 4;
