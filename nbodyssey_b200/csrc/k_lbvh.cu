@@ -737,7 +737,8 @@ __device__ __forceinline__ int clz_k(uint64_t x) { return __clzll((long long)x);
 // bit for bit).
 //
 // Levels.  A CTA takes a contiguous run of leaves and a sequence of "items"
-// separated by splits: at the first level the items are its 1024 leaves, at
+// separated by splits: at the first level the items are its leaves (256 to
+// 1,024), at
 // later levels the finished subtrees that the CTAs below left between the
 // splits they could not close.  At a split the first of the two children to
 // arrive parks its cell in shared memory and stops, the second merges both
@@ -752,11 +753,15 @@ __device__ __forceinline__ int clz_k(uint64_t x) { return __clzll((long long)x);
 // (kLevelItems - 1) / segment CTAs' segments per CTA; the level with one CTA
 // closes the root.
 // ---------------------------------------------------------------------------
-constexpr int kLeafGroup = 1024;     // leaves per CTA at the first level
-constexpr int kLevelThreads = 512;
-constexpr int kLevelItems = 2048;    // capacity of a later level's CTA
+constexpr int kLevelThreads = 512;     // later levels
+constexpr int kLevelItems = 2048;      // capacity of a later level's CTA
 constexpr int kSplitEmpty = -1;
 constexpr int kSplitDone = -2;
+// d of the missing split left of the tree's first leaf and right of its last
+// (real ones are >= 0): with them a node joins to the right exactly when the d
+// on its right is the larger
+constexpr int kDeltaFirst = -1;
+constexpr int kDeltaLast = -2;
 
 __host__ __device__ constexpr int level_seg(int key_bits) {
   return key_bits == 63 ? 192 : 128;
@@ -928,11 +933,11 @@ struct LevelSmem {
   double4* sum;    // [cap] cells by slot
   float4* lo;
   float4* hi;
-  int4* meta;      // [cap] (lo, hi, split leaf, Karras id) of a node formed
-                   // here, Karras id -1 for an item
+  int4* meta;      // [cap] (first item, last item, split) of a node formed
+                   // here, first item -1 for an item
   int* pos;        // [cap] leaf position of split k
-  int* delta;      // [cap + 1] delta[k + 1] = d(split k), delta[0] = d of the
-                   // split left of the run
+  int* delta;      // [cap + 1] delta[i] = d of the split left of item i (and
+                   // right of item i - 1)
   int* exch;       // [cap] far item of the first arrival at split k
   unsigned* list;  // [2][cap] pending arrivals (ia | ib << 16)
   int* scan;       // [40]
@@ -988,78 +993,90 @@ __device__ __forceinline__ void list_push(const LevelSmem& sm, int* count, int w
   if (push) sm.list[which * cap + base + __popc(mask & ((1u << lane) - 1u))] = v;
 }
 
-// A node over items [ia, ib] (leaves [lo, hi], cell c, formed here or an
-// item) that has just been finished: the root and frontier nodes are written
-// out; any other parks its cell in its slot and becomes a pending arrival.
-// Slot = the node's Karras id in item space (right end if it joins to the
-// right, left end otherwise); an item and a node formed later share a slot
-// only when the item is below the node, and the node is written after the
-// item's cell was read.  Returns whether it parked.
+// A node over items [ia, ib] with d values dl and dr beside it, split after
+// item sc (cell c, formed here or an item), that has just been finished: the
+// root and frontier nodes are written out; any other parks its cell in its
+// slot and becomes a pending arrival.  Slot = the node's Karras id in item space
+// (right end if it joins to the right, left end otherwise); an item and a node
+// formed later share a slot only when the item is below the node, and the node
+// is written after the item's cell was read.  Returns whether it parked.
 __device__ __forceinline__ bool finish_node(const TreeView& a, const LevelSmem& sm,
-                                            const Run& run, int ia, int ib, int lo,
-                                            int hi, int sc, bool formed, const Cell& c) {
+                                            const Run& run, int ia, int ib, int dl, int dr,
+                                            int sc, bool formed, const Cell& c) {
   const int ni = a.n - 1;
-  if (lo == 0 && hi == ni) {   // the root: this run is the whole tree
-    write_node(a, 0, lo, hi, sc, c);
+  if (dl == kDeltaFirst && dr == kDeltaLast) {   // the root: this run is the whole tree
+    if (formed) write_node(a, 0, 0, ni, sm.pos[sc], c);
+    else raise_err(a.err(), NB_DEVERR_TREE);   // only after a failed sort
     if (int* par = a.parent()) par[0] = -1;
     return false;
   }
-  const bool right = lo == 0 || (hi != ni && sm.delta[ib + 1] > sm.delta[ia]);
-  const int kid = right ? hi : lo;
+  const bool right = dr > dl;
   const int k = right ? ib : ia - 1;
   if (k < 0 || k >= run.local) {   // parent split on the run's boundary
     if (formed) {
-      write_node(a, kid, lo, hi, sc, c);
+      const int lo = run.item_lo(sm, ia), hi = run.item_hi(sm, ib, ni);
+      const int kid = right ? hi : lo;
+      write_node(a, kid, lo, hi, sm.pos[sc], c);
       store_cell(a, kid, c);
     }
     return false;
   }
   const int slot = right ? ib : ia;
   put_cell(sm, slot, c);
-  if (formed) sm.meta[slot] = make_int4(lo, hi, sc, kid);
+  if (formed) sm.meta[slot] = make_int4(ia, ib, sc, 0);
   return true;
 }
 
 // One pending arrival (items [ia, ib], parked in its slot) climbs until it
-// is the first at a split or finishes.  acq_rel: the exchange publishes this
-// thread's slot writes and acquires the sibling's.
+// is the first at a split or finishes.  PEEK (later levels, whose long climbs
+// collect small subtrees): a node that finds its sibling already there takes it
+// with a load, and only one that finds the split empty needs the exchange; at
+// the leaves, where half of all arrivals are first, the extra load costs more.
+// acq_rel: the exchange publishes this thread's slot writes and acquires the
+// sibling's, as does the load.  What bounds a step is its chain of shared-memory
+// latencies, so nothing else is on it: d values instead of leaf positions
+// decide the direction, and node records are written by the sweep.
+template <bool PEEK>
 __device__ __forceinline__ void climb_arrival(const TreeView& a, const LevelSmem& sm,
-                                              const Run& run, unsigned d) {
-  const int ni = a.n - 1;
-  int ia = (int)(d & 0xffffu), ib = (int)(d >> 16);
-  int lo = run.item_lo(sm, ia), hi = run.item_hi(sm, ib, ni);
-  bool right = lo == 0 || (hi != ni && sm.delta[ib + 1] > sm.delta[ia]);
-  Cell c = get_cell(sm, right ? ib : ia);
+                                              const Run& run, unsigned v) {
+  int ia = (int)(v & 0xffffu), ib = (int)(v >> 16);
+  int dl = sm.delta[ia], dr = sm.delta[ib + 1];
+  Cell c = get_cell(sm, dr > dl ? ib : ia);
   for (int guard = 0; guard <= run.items; ++guard) {
+    const bool right = dr > dl;
     const int k = right ? ib : ia - 1;
     cuda::atomic_ref<int, cuda::thread_scope_block> word(sm.exch[k]);
-    const int other = word.exchange(right ? ia : ib, cuda::memory_order_acq_rel);
-    if (other == kSplitEmpty) return;
+    int other = PEEK ? word.load(cuda::memory_order_acquire) : kSplitEmpty;
+    if (other == kSplitEmpty) {
+      other = word.exchange(right ? ia : ib, cuda::memory_order_acq_rel);
+      if (other == kSplitEmpty) return;
+    }
     if (other < 0 || other >= run.items || (right ? other <= k : other > k)) break;
     const Cell o = get_cell(sm, right ? k + 1 : k);
     sm.exch[k] = kSplitDone;
     if (right) {
       ib = other;
-      hi = run.item_hi(sm, other, ni);
+      dr = sm.delta[other + 1];
     } else {
       ia = other;
-      lo = run.item_lo(sm, other);
+      dl = sm.delta[other];
     }
     c = merge(c, o);
-    if (!finish_node(a, sm, run, ia, ib, lo, hi, sm.pos[k], true, c)) return;
-    right = lo == 0 || (hi != ni && sm.delta[ib + 1] > sm.delta[ia]);
+    if (!finish_node(a, sm, run, ia, ib, dl, dr, k, true, c)) return;
   }
   raise_err(a.err(), NB_DEVERR_TREE);
 }
 
 // Later levels hold 2048 items (196 KB of shared memory): one CTA per SM, so
 // they may use twice the registers of the first level's two CTAs.
-template <typename K, bool FIRST>
-__global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(LevelArgs args) {
+// G: leaves per CTA of a first level, 0 for a later one; T threads.
+template <typename K, int G, int T>
+__global__ void __launch_bounds__(T, G ? 1024 / T : 1) k_build_level(LevelArgs args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_release();
   chain_wait();
-  constexpr int C = FIRST ? kLeafGroup : kLevelItems;
+  constexpr bool FIRST = G > 0;
+  constexpr int C = FIRST ? G : kLevelItems;
   const LevelSmem sm(smem_raw, C);
   // this CTA's tree, its group index there, its input segments [sfirst,
   // sfirst + scount) and whether it hands open splits to the next level
@@ -1087,14 +1104,14 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
   Run run;
   if (FIRST) {
     const K* __restrict__ keys = static_cast<const K*>(p.keys) + sbase;
-    run.A = g * kLeafGroup;
-    run.B = min(n, run.A + kLeafGroup);
+    run.A = g * G;
+    run.B = min(n, run.A + G);
     run.M = run.B < n ? run.B - run.A : run.B - run.A - 1;
-    for (int k = tid; k < run.M; k += kLevelThreads) {
+    for (int k = tid; k < run.M; k += T) {
       sm.pos[k] = run.A + k;
       sm.delta[k + 1] = split_delta(keys, run.A + k);
     }
-    if (tid == 0) sm.delta[0] = run.A > 0 ? split_delta(keys, run.A - 1) : -1;
+    if (tid == 0) sm.delta[0] = run.A > 0 ? split_delta(keys, run.A - 1) : kDeltaFirst;
   } else {
     const int r0 = sfirst, r1 = sfirst + scount;
     if (warp == 0) {   // segment offsets (fan <= 32)
@@ -1108,7 +1125,7 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
       sm.scan[lane] = incl - c;
       if (lane == 31) sm.scan[32] = incl;
       if (lane == 0) {   // the last entry below is the split left of this run
-        int d = -1;
+        int d = kDeltaFirst;
         if (g > 0) {
           const int cp = min(p.in_count[r0 - 1], p.seg);
           if (cp > 0) d = p.in_seg[(size_t)(r0 - 1) * p.seg + cp - 1].y;
@@ -1119,7 +1136,7 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
     __syncthreads();
     run.M = sm.scan[32];
     // one warp per segment
-    for (int r = r0 + warp; r < r1; r += kLevelThreads / 32) {
+    for (int r = r0 + warp; r < r1; r += T / 32) {
       const int off = sm.scan[r - r0];
       const int c = sm.scan[r - r0 + 1] - off;
       for (int e = lane; e < c; e += 32) {
@@ -1134,27 +1151,28 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
   }
   run.items = run.B < n ? run.M : run.M + 1;
   run.local = run.B < n ? run.M - 1 : run.M;
-  for (int k = tid; k < run.M; k += kLevelThreads) sm.exch[k] = kSplitEmpty;
-  for (int j = tid; j < run.items; j += kLevelThreads) sm.meta[j].w = -1;
+  for (int k = tid; k < run.M; k += T) sm.exch[k] = kSplitEmpty;
+  for (int j = tid; j < run.items; j += T) sm.meta[j].x = -1;
+  if (tid == 0 && run.B >= n) sm.delta[run.items] = kDeltaLast;
   int* count = sm.scan + 34;   // three rotating list counters
   if (tid < 3) count[tid] = 0;
   __syncthreads();
 
   // round 0: every item parks its cell and becomes a pending arrival
-  for (int base = 0; base < run.items; base += kLevelThreads) {
+  for (int base = 0; base < run.items; base += T) {
     const int j = base + tid;
     bool push = false;
     if (j < run.items) {
       const int lo = run.item_lo(sm, j), hi = run.item_hi(sm, j, ni);
+      const int dl = sm.delta[j], dr = sm.delta[j + 1];
+      const bool right = dr > dl;
       Cell c;
       if (FIRST || lo == hi) {
         c = leaf_cell(a.ps(), lo);
         if (FIRST && ni > 0) {   // the leaf's half of its parent's pair record
-          const bool right = lo == 0 || (hi != ni && sm.delta[j + 1] > sm.delta[j]);
           write_pair_half(a, right ? lo : lo - 1, right ? 0 : 1, a.ps()[lo], -1.f, -1);
         }
       } else {   // a subtree finished below: its Karras id follows its direction
-        const bool right = lo == 0 || (hi != ni && sm.delta[j + 1] > sm.delta[j]);
         const int kid = right ? hi : lo;
         if (kid < ni) {
           c = load_cell(a, kid);
@@ -1163,7 +1181,7 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
           c = leaf_cell(a.ps(), lo);
         }
       }
-      push = finish_node(a, sm, run, j, j, lo, hi, -1, false, c);
+      push = finish_node(a, sm, run, j, j, dl, dr, -1, false, c);
     }
     list_push(sm, &count[0], 0, C, push, (unsigned)j | ((unsigned)j << 16));
   }
@@ -1178,20 +1196,20 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
   for (int round = 0; round <= run.items; ++round) {
     const int L = count[round % 3];
     if (L == 0) break;
-    if (L <= kLevelThreads) {
-      if (tid < L) climb_arrival(a, sm, run, sm.list[cur * C + tid]);
+    if (L <= T) {
+      if (tid < L) climb_arrival<!FIRST>(a, sm, run, sm.list[cur * C + tid]);
       break;
     }
     if (tid == 0) count[(round + 2) % 3] = 0;
-    for (int base = 0; base < L; base += kLevelThreads) {
+    for (int base = 0; base < L; base += T) {
       const int i = base + tid;
       bool push = false;
       unsigned v = 0;
       if (i < L) {
         const unsigned d = sm.list[cur * C + i];
         int ia = (int)(d & 0xffffu), ib = (int)(d >> 16);
-        int lo = run.item_lo(sm, ia), hi = run.item_hi(sm, ib, ni);
-        const bool right = lo == 0 || (hi != ni && sm.delta[ib + 1] > sm.delta[ia]);
+        int dl = sm.delta[ia], dr = sm.delta[ib + 1];
+        const bool right = dr > dl;
         const int k = right ? ib : ia - 1;
         const int other = atomicExch(&sm.exch[k], right ? ia : ib);
         if (other != kSplitEmpty) {
@@ -1203,12 +1221,12 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
             sm.exch[k] = kSplitDone;
             if (right) {
               ib = other;
-              hi = run.item_hi(sm, other, ni);
+              dr = sm.delta[other + 1];
             } else {
               ia = other;
-              lo = run.item_lo(sm, other);
+              dl = sm.delta[other];
             }
-            push = finish_node(a, sm, run, ia, ib, lo, hi, sm.pos[k], true, merge(mine, o));
+            push = finish_node(a, sm, run, ia, ib, dl, dr, k, true, merge(mine, o));
             v = (unsigned)ia | ((unsigned)ib << 16);
           }
         }
@@ -1220,22 +1238,26 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
   }
   __syncthreads();
   // node records of the nodes formed here, in slot order
-  for (int j = tid; j < run.items; j += kLevelThreads) {
+  for (int j = tid; j < run.items; j += T) {
     const int4 m = sm.meta[j];
-    if (m.w >= 0) write_node(a, m.w, m.x, m.y, m.z, get_cell(sm, j));
+    if (m.x < 0) continue;
+    const int lo = run.item_lo(sm, m.x), hi = run.item_hi(sm, m.y, ni);
+    const int kid = sm.delta[m.y + 1] > sm.delta[m.x] ? hi : lo;
+    write_node(a, kid, lo, hi, sm.pos[m.z], get_cell(sm, j));
   }
   if (!out) return;
   // a formed child waiting at an open split hands its cell to the next level
-  for (int k = tid; k < run.local; k += kLevelThreads) {
+  for (int k = tid; k < run.local; k += T) {
     const int e = sm.exch[k];
     if (e < 0) continue;
     const bool left = e <= k;   // the waiting child covers items [e, k]
     if (left ? e == k : e == k + 1) continue;   // a single item: stored below
     const int slot = left ? k : k + 1;
-    store_cell(a, sm.meta[slot].w, get_cell(sm, slot));
+    const int4 m = sm.meta[slot];
+    store_cell(a, left ? run.item_hi(sm, m.y, ni) : run.item_lo(sm, m.x), get_cell(sm, slot));
   }
   // open splits in order: (position, delta) into this CTA's segment
-  const int chunk = (run.M + kLevelThreads - 1) / kLevelThreads;
+  const int chunk = (run.M + T - 1) / T;
   const int k0 = min(run.M, tid * chunk), k1 = min(run.M, k0 + chunk);
   int cnt = 0;
   for (int k = k0; k < k1; ++k) cnt += (k >= run.local || sm.exch[k] != kSplitDone);
@@ -1248,7 +1270,7 @@ __global__ void __launch_bounds__(kLevelThreads, FIRST ? 2 : 1) k_build_level(Le
   if (lane == 31) sm.scan[warp] = incl;   // the segment offsets are no longer read
   __syncthreads();
   int base = 0, total = 0;
-  for (int w = 0; w < kLevelThreads / 32; ++w) {
+  for (int w = 0; w < T / 32; ++w) {
     const int v = sm.scan[w];
     if (w < warp) base += v;
     total += v;
@@ -1284,38 +1306,73 @@ static LevelArgs level_args(Workspace& w, const StepArgs& a) {
   return b;
 }
 
+// Launches of later levels above `groups` groups.
+static int later_levels(int groups, int fan) {
+  int lv = 0;
+  for (; groups > 1; ++lv) groups = (groups + fan - 1) / fan;
+  return lv;
+}
+
+// Leaves per CTA at the first level: the fewest that need no more levels than
+// groups of 1,024 do.  A first level lasts as long as its CTAs' climbs, which
+// grow with the group, and a later level about 10 us whatever it holds.  Both
+// levels together: 36 us against 46 at n = 20,011 (256 leaves), 46 / 48 at 100,000
+// (512), 110 / 119 at 1M (512).
+static int leaf_group(int n, int fan) {
+  const int lv = later_levels((n + 1023) / 1024, fan);
+  for (int g : {256, 512})
+    if (later_levels((n + g - 1) / g, fan) <= lv) return g;
+  return 1024;
+}
+
 size_t build_seg_entries(int cap) {
-  return (size_t)((cap + kLeafGroup - 1) / kLeafGroup) * level_seg(63);
+  return ((size_t)cap / 256 + 1) * level_seg(63);   // the smallest groups
+}
+
+template <typename K>
+static int launch_first_level(int group, int groups, const LevelArgs& b, cudaStream_t st,
+                              bool chained) {
+  auto go = [&](auto kernel, int G, int T) {
+    const int smem = (int)level_smem(G);
+    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (chained) return launch_chained(kernel, groups, T, smem, st, b);
+    kernel<<<groups, T, smem, st>>>(b);
+    NB_CUDA(cudaGetLastError());
+    return NB_OK;
+  };
+  // a thread per leaf while every CTA is resident at once, half as many (twice
+  // the groups in flight) above
+  if (groups * group <= 1024 * device_sm_count()) {
+    if (group == 256) return go(k_build_level<K, 256, 256>, 256, 256);
+    if (group == 512) return go(k_build_level<K, 512, 512>, 512, 512);
+  }
+  if (group == 256) return go(k_build_level<K, 256, 128>, 256, 128);
+  if (group == 512) return go(k_build_level<K, 512, 256>, 512, 256);
+  return go(k_build_level<K, 1024, 512>, 1024, 512);
 }
 
 // First level: leaf groups (the bottom of the tree, most of its nodes).
 int launch_build(Workspace& w, const StepArgs& a, cudaStream_t st) {
   LevelArgs b = level_args(w, a);
-  const int groups = (a.n + kLeafGroup - 1) / kLeafGroup;
+  const int group = leaf_group(a.n, b.fan);
+  const int groups = (a.n + group - 1) / group;
   if (groups > 1) {
     b.out_seg = w.seg[0];
     b.out_count = w.seg_count[0];
   }
-  const int smem = (int)level_smem(kLeafGroup);
-  if (a.key_bits == 63) {
-    NB_CUDA(cudaFuncSetAttribute(k_build_level<uint64_t, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    return launch_chained(k_build_level<uint64_t, true>, groups, kLevelThreads, smem, st, b);
-  } else {
-    NB_CUDA(cudaFuncSetAttribute(k_build_level<uint32_t, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    return launch_chained(k_build_level<uint32_t, true>, groups, kLevelThreads, smem, st, b);
-  }
+  if (a.key_bits == 63) return launch_first_level<uint64_t>(group, groups, b, st, true);
+  return launch_first_level<uint32_t>(group, groups, b, st, true);
 }
 
 // Later levels: the tree above the leaf groups, up to the root.
 int launch_com(Workspace& w, const StepArgs& a, cudaStream_t st) {
   LevelArgs b = level_args(w, a);
   const int smem = (int)level_smem(kLevelItems);
-  NB_CUDA(cudaFuncSetAttribute(k_build_level<uint32_t, false>,
+  NB_CUDA(cudaFuncSetAttribute(k_build_level<uint32_t, 0, kLevelThreads>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  int groups = (a.n + kLeafGroup - 1) / kLeafGroup;
-  long long span = kLeafGroup;
+  const int group = leaf_group(a.n, b.fan);
+  int groups = (a.n + group - 1) / group;
+  long long span = group;
   int p = 0;
   while (groups > 1) {
     const int next = (groups + b.fan - 1) / b.fan;
@@ -1325,7 +1382,7 @@ int launch_com(Workspace& w, const StepArgs& a, cudaStream_t st) {
     b.in_span = span;
     b.out_seg = next > 1 ? w.seg[p ^ 1] : nullptr;
     b.out_count = next > 1 ? w.seg_count[p ^ 1] : nullptr;
-    NB_TRY(launch_chained(k_build_level<uint32_t, false>, next, kLevelThreads, smem, st, b));
+    NB_TRY(launch_chained(k_build_level<uint32_t, 0, kLevelThreads>, next, kLevelThreads, smem, st, b));
     groups = next;
     span *= b.fan;
     p ^= 1;
@@ -1430,6 +1487,10 @@ int launch_ens_sort(EnsArgs& e, cudaStream_t st) {
 // has one run.  The 64-bit keys (sim << 30) | morton30 give the same
 // Cartesian tree as the simulation's own keys (the shared prefix shifts every
 // d by 32), so each tree equals the one the simulation builds alone.
+// One group size for all trees of a batch: with 512, small trees get a level
+// more (24 encounters of up to 16,384 particles 189 -> 194 us a step, 64 of up to
+// 32,768 426 -> 418).
+constexpr int kEnsLeafGroup = 1024;
 int plan_build(const SimDesc* sims, int nsims, BuildPlan& plan) {
   plan.levels = 0;
   plan.runs.clear();
@@ -1437,7 +1498,7 @@ int plan_build(const SimDesc* sims, int nsims, BuildPlan& plan) {
   int live = 0;
   for (int s = 0; s < nsims; ++s)
     if (sims[s].active && sims[s].n >= 2 && sims[s].force == NB_FORCE_BH) {
-      groups[s] = (sims[s].n + kLeafGroup - 1) / kLeafGroup;
+      groups[s] = (sims[s].n + kEnsLeafGroup - 1) / kEnsLeafGroup;
       ++live;
     }
   if (!live) return NB_OK;
@@ -1470,7 +1531,7 @@ int plan_build(const SimDesc* sims, int nsims, BuildPlan& plan) {
 }
 
 size_t plan_seg_entries(int slots, int nsims) {
-  return ((size_t)slots / kLeafGroup + (size_t)nsims + 1) * level_seg(30);
+  return ((size_t)slots / kEnsLeafGroup + (size_t)nsims + 1) * level_seg(30);
 }
 
 int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st) {
@@ -1487,7 +1548,7 @@ int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st) 
   b.fan = level_fan(30);
   b.err = e.err;
   b.sims = e.sims;
-  long long span = kLeafGroup;
+  long long span = kEnsLeafGroup;
   for (int lv = 0; lv < plan.levels; ++lv) {
     const int runs = plan.count[lv];
     if (runs == 0) continue;
@@ -1501,15 +1562,12 @@ int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st) 
     b.out_seg = lv + 1 < plan.levels ? e.seg[lv & 1] : nullptr;
     b.out_count = lv + 1 < plan.levels ? e.seg_count[lv & 1] : nullptr;
     if (lv == 0) {
-      const int smem = (int)level_smem(kLeafGroup);
-      NB_CUDA(cudaFuncSetAttribute(k_build_level<uint64_t, true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      k_build_level<uint64_t, true><<<runs, kLevelThreads, smem, st>>>(b);
+      NB_TRY(launch_first_level<uint64_t>(kEnsLeafGroup, runs, b, st, false));
     } else {
       const int smem = (int)level_smem(kLevelItems);
-      NB_CUDA(cudaFuncSetAttribute(k_build_level<uint32_t, false>,
+      NB_CUDA(cudaFuncSetAttribute(k_build_level<uint32_t, 0, kLevelThreads>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      k_build_level<uint32_t, false><<<runs, kLevelThreads, smem, st>>>(b);
+      k_build_level<uint32_t, 0, kLevelThreads><<<runs, kLevelThreads, smem, st>>>(b);
     }
     NB_CUDA(cudaGetLastError());
   }
@@ -1521,8 +1579,12 @@ int warm_lbvh_kernels() {
                   k_sort_cluster<uint32_t>, k_sort_cluster<uint64_t>,
                   k_sort_pass<uint32_t, kSortMid>, k_sort_pass<uint32_t, kSortLast>,
                   k_sort_pass<uint64_t, kSortMid>, k_sort_pass<uint64_t, kSortLast>,
-                  k_sort_pass<uint64_t, kSortLastEnsemble>, k_build_level<uint32_t, true>,
-                  k_build_level<uint64_t, true>, k_build_level<uint32_t, false>);
+                  k_sort_pass<uint64_t, kSortLastEnsemble>, k_build_level<uint32_t, 256, 256>,
+                  k_build_level<uint32_t, 256, 128>, k_build_level<uint32_t, 512, 512>,
+                  k_build_level<uint32_t, 512, 256>, k_build_level<uint32_t, 1024, 512>,
+                  k_build_level<uint64_t, 256, 256>, k_build_level<uint64_t, 256, 128>,
+                  k_build_level<uint64_t, 512, 512>, k_build_level<uint64_t, 512, 256>,
+                  k_build_level<uint64_t, 1024, 512>, k_build_level<uint32_t, 0, kLevelThreads>);
 }
 
 }  // namespace nb
