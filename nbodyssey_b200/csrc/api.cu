@@ -77,6 +77,7 @@ int warm_kernels() {
   NB_TRY(warm_walk_kernels());
   NB_TRY(warm_allpairs_kernels());
   NB_TRY(warm_allpairs_sym_kernels());
+  NB_TRY(warm_allpairs_small_kernels());
   NB_TRY(warm_fns(k_differ));
   done[dev] = true;
   return NB_OK;
@@ -202,6 +203,7 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
 }
 
 int ws_reserve_naive(Workspace& w, int n) {
+  if (n < kSymMin) return ws_basic(w);   // no scratch
   if (allpairs_sym(n)) return ws_reserve_allpairs_sym(w, n);
   return ws_reserve_allpairs(w, n, allpairs_geometry(n));
 }
@@ -325,9 +327,9 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
     return mark(pm, NB_PHASE_WALK, st);
   }
   if (force == NB_FORCE_NAIVE) {
-    // the pairs-once kernel reads the positions themselves: nothing to pack
-    const bool sym = allpairs_sym(a.n);
-    if (!sym || a.kick_drift) NB_TRY(launch_prep(w, a, false, !sym, st));
+    // up to kSymMax the kernels read the positions themselves: nothing to pack
+    const bool pack = a.n > kSymMax;
+    if (pack || a.kick_drift) NB_TRY(launch_prep(w, a, false, pack, st));
     if (a.after_prep) NB_CUDA(cudaEventRecord(a.after_prep, st));
     NB_TRY(mark(pm, NB_PHASE_PREP, st));
     NB_TRY(launch_allpairs(w, a, st));

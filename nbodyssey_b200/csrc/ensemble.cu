@@ -242,6 +242,7 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
       if ((rc = ens_alloc(h, &ap.d_src_off, (size_t)nsims)) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_counter, 6)) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.sym.d_table, ap.sym.bytes())) != NB_OK) break;
+      if ((rc = ens_alloc(h, &ap.d_small, ap.small.size())) != NB_OK) break;
     }
     {
       BuildRun* runs = nullptr;
@@ -323,6 +324,7 @@ int nb_ensemble_kernels_per_step(const nb_ensemble* h, int* kernels) {
   }
   if (!h->ap.groups.empty()) k += 1 + (int)h->ap.groups.size();   // pack + queues
   k += 2 * (int)h->ap.sym.passes.size();   // pairs-once items and their reduction
+  k += h->ap.small.empty() ? 0 : 1;
   *kernels = k;
   return NB_OK;
 }

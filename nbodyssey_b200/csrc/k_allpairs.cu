@@ -333,6 +333,17 @@ int launch_allpairs_geom(Workspace& w, const StepArgs& s, const APGeom& g,
 }
 
 int launch_allpairs(Workspace& w, const StepArgs& s, cudaStream_t st) {
+  if (s.n < kSymMin) {
+    APArgs a{};
+    a.n = s.n;
+    a.pos = s.pos;
+    a.eps2 = s.eps2;
+    a.G = s.G;
+    a.half_dt = s.half_dt;
+    a.acc = s.acc;
+    a.vel = s.kick_after ? s.vel : nullptr;
+    return launch_allpairs_small(a, st);
+  }
   if (allpairs_sym(s.n))
     return launch_allpairs_sym(s.n, s.pos, s.acc, s.kick_after ? s.vel : nullptr, s.eps2, s.G,
                                s.half_dt, w.part, (size_t)w.part_cap, st);
@@ -396,6 +407,7 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
   ap.groups.clear();
   ap.src_off.assign(nsims, -1);
   ap.sym.clear();
+  ap.small.clear();
   // the tables of the pairs-once simulations, whole when they may be
   size_t whole = 0;
   for (int s = 0; s < nsims; ++s)
@@ -431,8 +443,13 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
       ap.sym.add(s, d, r, size);
       continue;
     }
-    ap.src_off[s] = (int)r;
-    todo.push_back({(int)ap.args.size(), g});
+    if (d.n < kSymMin) {
+      for (int t = 0; t < d.n; t += small_batch_targets())
+        ap.small.push_back(make_int2((int)ap.args.size(), t));
+    } else {
+      ap.src_off[s] = (int)r;
+      todo.push_back({(int)ap.args.size(), g});
+    }
     ap.args.push_back(a);
     ap.sim.push_back(s);
     ap.region.push_back(r);
@@ -479,6 +496,9 @@ int bind_ens_allpairs(EnsAllPairs& ap, const SimDesc* sims, int nsims, const Ens
   if (!ap.items.empty())
     NB_CUDA(cudaMemcpyAsync(ap.d_items, ap.items.data(), sizeof(int4) * ap.items.size(),
                             cudaMemcpyHostToDevice, st));
+  if (!ap.small.empty())
+    NB_CUDA(cudaMemcpyAsync(ap.d_small, ap.small.data(), sizeof(int2) * ap.small.size(),
+                            cudaMemcpyHostToDevice, st));
   NB_CUDA(cudaMemcpyAsync(ap.d_src_off, ap.src_off.data(), sizeof(int) * nsims,
                           cudaMemcpyHostToDevice, st));
   return ap.sym.bind(sims, e, ap.d_pool, st);
@@ -491,6 +511,9 @@ static void launch_queue(const APQueue& q, int grid, cudaStream_t st) {
 
 int launch_ens_allpairs(const EnsArgs& e, const EnsAllPairs& ap, cudaStream_t st) {
   NB_TRY(ap.sym.launch(e, st));
+  if (!ap.small.empty())
+    NB_TRY(launch_allpairs_small_batch(ap.d_args, (int)ap.args.size(), ap.d_small,
+                                       (int)ap.small.size(), e.kick_after, e.err, st));
   if (ap.groups.empty()) return NB_OK;
   k_ens_pack<<<(e.nblocks * 32 + 255) / 256, 256, 0, st>>>(e, ap.d_src_off, ap.d_pool);
   NB_CUDA(cudaGetLastError());

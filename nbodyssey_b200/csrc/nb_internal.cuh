@@ -300,6 +300,14 @@ struct APArgs {
   unsigned* err;
 };
 
+// All-pairs for n below kSymMin (k_allpairs_small.cu): reads `pos` alone of the
+// sources' fields.
+int launch_allpairs_small(const APArgs& a, cudaStream_t st);
+int launch_allpairs_small_batch(const APArgs* args, int nargs, const int2* items, int nitems,
+                                bool kick, unsigned* err, cudaStream_t st);
+int small_batch_targets();   // targets of one batch item
+int warm_allpairs_small_kernels();
+
 // The persistent all-pairs launch over many simulations' work items.
 struct APQueue {
   const APArgs* sims;     // per-simulation arguments (pointers into its slots)
@@ -328,10 +336,11 @@ int launch_allpairs_geom(Workspace& w, const StepArgs& a, const APGeom& g,
 
 // All-pairs with each unordered pair evaluated once (k_allpairs_sym.cu): a
 // function of n alone (order of the sums included), whatever the tuning table.
-// A step of kSymMin particles takes 14.4 us against 20.5 with the tiled kernel;
-// below, batches of small simulations keep the tiled kernel's work queue, and
-// kSymMax bounds the tables that a batch's plan uploads.
-constexpr int kSymMin = 2048;
+// Below kSymMin one launch without any summing up is faster (a step of 2,560
+// particles 12.5 us against 14.4, of 4,096 17.3 against 16.4; batches gain from it
+// earlier, 64 of 2,100 150 us against 117); kSymMax bounds the tables that a batch's
+// plan uploads.
+constexpr int kSymMin = 2560;
 constexpr int kSymMax = 1 << 20;
 bool allpairs_sym(int n);
 struct SymGeom {
@@ -503,6 +512,8 @@ struct EnsAllPairs {
   std::vector<int> src_off;    // per simulation: pool offset of its packed
                                // sources, -1 for one without any
   SymPlan sym;                 // the simulations of the pairs-once kernel
+  std::vector<int2> small;     // (entry, first target) of the small ones' items
+  int2* d_small = nullptr;
   // device (owned by the batch)
   float4* d_pool = nullptr;
   APArgs* d_args = nullptr;

@@ -100,6 +100,7 @@ struct nb_server {
   std::vector<size_t> ap_region_cap; // by sim id: region size (float4)
   EnsAllPairs ap;
   size_t ap_items_cap = 0;
+  size_t ap_small_cap = 0;           // small simulations' items
   size_t ap_sym_cap = 0;             // bytes of the pairs-once table
   bool any_tree = false;
   std::vector<int> walk_items[2];    // the walk queue (host copy)
@@ -375,6 +376,15 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
       NB_CUDA(cudaMalloc(&s->ap.d_items, sizeof(int4) * cap));
       s->ap_items_cap = cap;
     }
+    if (s->ap.small.size() > s->ap_small_cap) {
+      NB_CUDA(cudaStreamSynchronize(s->stream));
+      if (s->ap.d_small) cudaFree(s->ap.d_small);
+      s->ap.d_small = nullptr;
+      s->ap_small_cap = 0;
+      const size_t cap = std::max(s->ap.small.size() * 2, (size_t)4096);
+      NB_CUDA(cudaMalloc((void**)&s->ap.d_small, sizeof(int2) * cap));
+      s->ap_small_cap = cap;
+    }
     if (s->ap.sym.bytes() > s->ap_sym_cap) {   // grow-only, rare
       NB_CUDA(cudaStreamSynchronize(s->stream));
       if (s->ap.sym.d_table) cudaFree(s->ap.sym.d_table);
@@ -642,6 +652,7 @@ int nb_server_destroy(nb_server* s) {
   for (void* p : s->dallocs) cudaFree(p);
   if (s->ap.d_items) cudaFree(s->ap.d_items);
   if (s->ap.sym.d_table) cudaFree(s->ap.sym.d_table);
+  if (s->ap.d_small) cudaFree(s->ap.d_small);
   if (s->h_frame) cudaFreeHost(s->h_frame);
   cudaStreamDestroy(s->stream);
   cudaStreamDestroy(s->side);

@@ -1,6 +1,7 @@
-"""The all-pairs kernel that evaluates each unordered pair once (n from 2,048
-on): tile and chunk edges, masses equal and not, ranges of scale, and passes
-over a scratch too small for the whole table of partials."""
+"""The all-pairs kernels: a warp per few targets below n = 2,560 (2 or 4
+targets a warp by size, 8 in a batch; sources in batches of 128), each unordered pair once
+from there on: tile and chunk edges, masses equal and not, ranges of scale, and
+passes over a scratch too small for the whole table of partials."""
 import numpy as np
 import pytest
 
@@ -23,9 +24,10 @@ def _forces(pos, eps=EPS):
         return sim.compute_forces()
 
 
-# the last of the tiled kernel, then both sides of every tile size and ragged
-# last tiles and chunks
-@pytest.mark.parametrize("n", [2047, 2048, 2049, 2304, 2305, 4097, 16384, 16385, 24576, 24577,
+# the small kernel's batches and target counts, then both sides of every tile
+# size and ragged last tiles and chunks
+@pytest.mark.parametrize("n", [127, 128, 129, 1184, 1185, 2047, 2048, 2049, 2304, 2305, 2559, 2560, 2561,
+                               4097, 8191, 8192, 8193, 8448, 8449, 16384, 16385, 24576, 24577,
                                65536, 65537, 131073])
 @pytest.mark.parametrize("masses", ["equal", "spread"])
 def test_sizes_vs_fp64(n, masses):
@@ -36,18 +38,18 @@ def test_sizes_vs_fp64(n, masses):
         pos[rng.choice(n, n // 50, replace=False), 3] = 0.0   # massless tracers
     acc = _forces(pos)
     assert np.all(acc[:, 3] == 0.0) and np.all(np.isfinite(acc))
-    tg = np.unique(np.concatenate([np.arange(300), np.arange(n - 300, n),
-                                   np.random.default_rng(1).choice(n, 600)]))
+    tg = np.unique(np.concatenate([np.arange(min(n, 300)), np.arange(max(0, n - 300), n),
+                                   np.random.default_rng(1).choice(n, min(n, 600))]))
     r = _rel(acc[tg, :3].astype(np.float64), O.allpairs_f64(pos, EPS, targets=tg))
     # the bounds the tiled kernel is held to (test_gpu_forces.py)
     assert np.median(r) < 2e-6 and np.percentile(r, 99) < 2e-5
 
 
+@pytest.mark.parametrize("n", [2500, 9000])
 @pytest.mark.parametrize("scale,mass", [(1e12, 1e30), (1e-10, 1e-6), (1e15, 1e33)])
-def test_scales(scale, mass):
+def test_scales(n, scale, mass):
     """The factor m / r^3 is built as (m / r) / r^2, so that lengths and
     masses far from 1 keep their digits (r^-3 alone would underflow)."""
-    n = 2500
     base, _ = ic.two_disks(n, seed=3)
     pos = base.copy()
     pos[:, :3] *= np.float32(scale)
