@@ -356,8 +356,13 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   return mark(pm, NB_PHASE_WALK, st);
 }
 
+// Waits for the stream (its error word is the last thing on it) and reports
+// what the kernels raised.
 static int check_device_error(Workspace& w, cudaStream_t st) {
-  if (!w.err) return NB_OK;
+  if (!w.err) {
+    NB_CUDA(cudaStreamSynchronize(st));
+    return NB_OK;
+  }
   NB_CUDA(cudaMemcpyAsync(w.h_err, w.err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   NB_CUDA(cudaStreamSynchronize(st));
   unsigned e = *w.h_err;
@@ -720,7 +725,6 @@ static int download(nb_sim* s, float* dst, const float4* src) {
   if (!s || !dst) return set_error(NB_ERR_INVALID, "NULL argument");
   NB_CUDA(cudaMemcpyAsync(dst, src, sizeof(float4) * s->n,
                           cudaMemcpyDeviceToHost, s->stream));
-  NB_CUDA(cudaStreamSynchronize(s->stream));
   return check_device_error(s->ws, s->stream);
 }
 
@@ -795,7 +799,6 @@ int nb_step_host(nb_sim* s, const float* pos4, const float* vel4, const float* a
   NB_CUDA(cudaMemcpyAsync(vel_out4, s->vel, b, cudaMemcpyDeviceToHost, s->stream));
   NB_CUDA(cudaMemcpyAsync(acc_out4, s->acc, b, cudaMemcpyDeviceToHost, s->stream));
   NB_CUDA(cudaStreamSynchronize(s->io_stream));
-  NB_CUDA(cudaStreamSynchronize(s->stream));
   return check_device_error(s->ws, s->stream);
 }
 
@@ -847,7 +850,6 @@ int nb_step_host_state(nb_sim* s, const float* pos4, const float* vel4, float* p
   NB_CUDA(cudaMemcpyAsync(pos_out4, s->pos, b, cudaMemcpyDeviceToHost, s->io_stream));
   NB_CUDA(cudaMemcpyAsync(vel_out4, s->vel, b, cudaMemcpyDeviceToHost, st));
   NB_CUDA(cudaStreamSynchronize(s->io_stream));
-  NB_CUDA(cudaStreamSynchronize(st));
   return check_device_error(s->ws, st);
 }
 
@@ -882,7 +884,6 @@ int nb_step(nb_sim* s, int nsteps) {
 
 int nb_sync(nb_sim* s) {
   if (!s) return set_error(NB_ERR_INVALID, "sim is NULL");
-  NB_CUDA(cudaStreamSynchronize(s->stream));
   return check_device_error(s->ws, s->stream);
 }
 
@@ -898,7 +899,6 @@ int nb_energy(nb_sim* s, double* e3, double* mom3) {
   if (pm) NB_TRY(mark(pm, NB_PHASE_ENERGY, s->stream));
   NB_CUDA(cudaMemcpyAsync(s->ws.h_eout, s->ws.eout, 6 * sizeof(double),
                           cudaMemcpyDeviceToHost, s->stream));
-  NB_CUDA(cudaStreamSynchronize(s->stream));
   NB_TRY(check_device_error(s->ws, s->stream));
   e3[0] = s->ws.h_eout[0];
   e3[1] = s->ws.h_eout[1];
@@ -1176,7 +1176,6 @@ int nb_total_energy_dev(nb_workspace* w, int n, const float* d_pos4,
                        p->eps * p->eps, p->G, st));
   NB_CUDA(cudaMemcpyAsync(w->ws.h_eout, w->ws.eout, 6 * sizeof(double),
                           cudaMemcpyDeviceToHost, st));
-  NB_CUDA(cudaStreamSynchronize(st));
   NB_TRY(check_device_error(w->ws, st));
   e3[0] = w->ws.h_eout[0];
   e3[1] = w->ws.h_eout[1];

@@ -31,6 +31,7 @@ struct nb_ensemble {
   std::vector<int> walk_items[2];   // the walk queue (host copy)
   Workspace ews;               // energy scratch
   double* d_energy = nullptr;  // [nsims][6]
+  unsigned* h_err = nullptr;   // pinned
   bool primed = false;
   bool any_tree = false;       // some simulation uses the tree pipeline
   bool use_graphs = true;
@@ -62,6 +63,7 @@ void ens_free(nb_ensemble* h) {
     if (ev) cudaEventDestroy(ev);
   for (void* p : h->allocs) cudaFree(p);
   ws_free(h->ews);
+  if (h->h_err) cudaFreeHost(h->h_err);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -123,10 +125,13 @@ int ens_capture(nb_ensemble* h) {
   return NB_OK;
 }
 
+// Waits for the stream (its error word is the last thing on it) and reports
+// what the kernels raised.
 int ens_device_error(nb_ensemble* h) {
-  unsigned v = 0;
-  NB_CUDA(cudaMemcpyAsync(&v, h->e.err, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+  NB_CUDA(cudaMemcpyAsync(h->h_err, h->e.err, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                          h->stream));
   NB_CUDA(cudaStreamSynchronize(h->stream));
+  const unsigned v = *h->h_err;
   if (v) {
     NB_CUDA(cudaMemsetAsync(h->e.err, 0, sizeof(unsigned), h->stream));
     NB_CUDA(cudaStreamSynchronize(h->stream));
@@ -257,6 +262,7 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     }
     if ((rc = ens_alloc(h, &h->d_energy, 6 * (size_t)nsims)) != NB_OK) break;
     cudaError_t ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
+    if (ce == cudaSuccess) ce = cudaMallocHost((void**)&h->h_err, sizeof(unsigned));
     if (ce != cudaSuccess) { rc = set_error(NB_ERR_CUDA, cudaGetErrorString(ce)); break; }
     cudaStream_t st = h->stream;
     // defined contents everywhere: zero state in the gaps, in-range indices
@@ -372,7 +378,6 @@ int nb_ensemble_set_graphs(nb_ensemble* h, int enable) {
 
 int nb_ensemble_sync(nb_ensemble* h) {
   if (!h) return set_error(NB_ERR_INVALID, "ensemble is NULL");
-  NB_CUDA(cudaStreamSynchronize(h->stream));
   return ens_device_error(h);
 }
 
@@ -386,7 +391,6 @@ int nb_ensemble_get_state(nb_ensemble* h, int sim, float* pos4, float* vel4) {
   if (vel4)
     NB_CUDA(cudaMemcpyAsync(vel4, h->e.vel + h->base[sim], bytes,
                             cudaMemcpyDeviceToHost, h->stream));
-  NB_CUDA(cudaStreamSynchronize(h->stream));
   return ens_device_error(h);
 }
 
@@ -395,7 +399,6 @@ int nb_ensemble_get_accelerations(nb_ensemble* h, int sim, float* acc4) {
   if (sim < 0 || sim >= h->nsims) return set_error(NB_ERR_NOTFOUND, "no such simulation");
   NB_CUDA(cudaMemcpyAsync(acc4, h->e.acc + h->base[sim], 16 * (size_t)h->n[sim],
                           cudaMemcpyDeviceToHost, h->stream));
-  NB_CUDA(cudaStreamSynchronize(h->stream));
   return ens_device_error(h);
 }
 
@@ -412,7 +415,6 @@ int nb_ensemble_energy(nb_ensemble* h, double* e3) {
   std::vector<double> buf(6 * (size_t)h->nsims);
   NB_CUDA(cudaMemcpyAsync(buf.data(), h->d_energy, buf.size() * sizeof(double),
                           cudaMemcpyDeviceToHost, h->stream));
-  NB_CUDA(cudaStreamSynchronize(h->stream));
   NB_TRY(ens_device_error(h));
   for (int s = 0; s < h->nsims; ++s)
     for (int c = 0; c < 3; ++c) e3[3 * s + c] = buf[6 * s + c];
