@@ -152,7 +152,7 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   NB_CUDA(cudaMemset(w.parent, 0xff, 2 * (size_t)cap * sizeof(int)));
   NB_CUDA(cudaMemset(w.nodes, 0, ni * sizeof(Node)));
   NB_CUDA(cudaMemset(w.pairs, 0, (size_t)cap * sizeof(PairRec)));
-  w.status_tiles = (cap + kSortTile - 1) / kSortTile;
+  w.status_tiles = sort_status_tiles(cap);
   size_t words = 8 * kSortRadix + 8 + (size_t)8 * w.status_tiles * kSortRadix;
   NB_TRY(dalloc(&w.hist, words));
   NB_CUDA(cudaMemset(w.hist, 0, words * sizeof(uint32_t)));

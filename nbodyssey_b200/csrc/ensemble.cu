@@ -221,7 +221,7 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     if ((rc = ens_alloc(h, &e.box_hi, S)) != NB_OK) break;
     if ((rc = ens_alloc(h, &e.bbox_min, 4 * (size_t)nsims)) != NB_OK) break;
     if ((rc = ens_alloc(h, &e.bbox_max, 4 * (size_t)nsims)) != NB_OK) break;
-    e.status_tiles = (b + kSortTile - 1) / kSortTile;
+    e.status_tiles = sort_status_tiles(b);
     const size_t words = 8 * kSortRadix + 8 + (size_t)8 * e.status_tiles * kSortRadix;
     if ((rc = ens_alloc(h, &e.hist, words)) != NB_OK) break;
     e.tile_ctr = e.hist + 8 * kSortRadix;

@@ -118,8 +118,8 @@ int launch_morton(Workspace& w, const StepArgs& a, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Onesweep LSD radix sort (Adinets & Merrill, 2022), 8-bit digits, stable.
 // Per pass one kernel: each CTA takes the next tile by ticket (so it only
-// waits on CTAs that are already running), ranks its keys with warp ballots
-// per digit bit, publishes its digit counts, resolves its global offsets by a
+// waits on CTAs that are already running), ranks its keys warp by warp,
+// publishes its digit counts, resolves its global offsets by a
 // decoupled look-back over earlier tiles (bounded waits), stages the tile in
 // digit order in shared memory and writes each digit's run contiguously.
 // ---------------------------------------------------------------------------
@@ -146,21 +146,7 @@ constexpr int kSortMid = 0;
 constexpr int kSortLast = 1;
 constexpr int kSortLastEnsemble = 2;
 
-// Lanes of the warp whose (valid) item has the same 8-bit digit: one ballot
-// per digit bit, so the cost does not grow with the number of distinct
-// digits in the warp.  Meaningful for lanes with ok set.
-__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool ok) {
-  uint32_t m = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const bool bit = (d >> b) & 1u;
-    const uint32_t v = __ballot_sync(0xffffffffu, bit);
-    m &= bit ? v : ~v;
-  }
-  return m;
-}
-
-template <typename K, int MODE>
+template <typename K, int MODE, int ITEMS>
 __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
     k_sort_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                 K* __restrict__ kout, uint32_t* __restrict__ vout, int n,
@@ -169,8 +155,10 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
                 const float4* __restrict__ pos, float4* __restrict__ pos_sorted,
                 const SimDesc* __restrict__ sims, int nsims) {
   constexpr int W = kSortThreads / 32;
+  constexpr int kSortTile = kSortThreads * ITEMS;
   static_assert(kSortThreads >= kSortRadix, "one thread per digit at least");
   __shared__ uint32_t s_wc[W][kSortRadix];
+  __shared__ uint32_t s_match[W][kSortRadix];
   __shared__ uint32_t s_base[kSortRadix];
   __shared__ uint32_t s_tex[kSortRadix];
   __shared__ uint32_t s_scan[W];
@@ -184,7 +172,10 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
   chain_release();
   chain_wait();
   if (tid == 0) s_tile = (int)atomicAdd(tile_ctr, 1u);
-  for (int i = tid; i < W * kSortRadix; i += kSortThreads) (&s_wc[0][0])[i] = 0u;
+  for (int i = tid; i < W * kSortRadix; i += kSortThreads) {
+    (&s_wc[0][0])[i] = 0u;
+    (&s_match[0][0])[i] = 0u;
+  }
 
   // threads [0, kSortRadix) own one digit each in the per-digit steps
   const bool dig = tid < kSortRadix;
@@ -203,12 +194,12 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
   const uint32_t gexcl = wofs + incl - h;
 
   const int tile = s_tile;
-  const long seg = (long)tile * kSortTile + (long)warp * (kSortItems * 32);
-  K key[kSortItems];
-  uint32_t val[kSortItems];
-  uint32_t rank[kSortItems];
+  const long seg = (long)tile * kSortTile + (long)warp * (ITEMS * 32);
+  K key[ITEMS];
+  uint32_t val[ITEMS];
+  uint32_t rank[ITEMS];
 #pragma unroll
-  for (int k = 0; k < kSortItems; ++k) {
+  for (int k = 0; k < ITEMS; ++k) {
     long idx = seg + k * 32 + lane;
     bool ok = idx < n;
     key[k] = ok ? kin[idx] : (K)0;
@@ -216,18 +207,25 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
   }
   const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
-  for (int k = 0; k < kSortItems; ++k) {
+  for (int k = 0; k < ITEMS; ++k) {
     long idx = seg + k * 32 + lane;
     bool ok = idx < n;
     uint32_t d = ok ? (uint32_t)((key[k] >> shift) & 0xffu) : 0u;
-    uint32_t peers = digit_peers(d, ok);
-    uint32_t old = 0;
+    // the lanes with this digit set their bits in its word; the first of them
+    // counts them and clears it (one ballot per digit bit took 10 % longer)
+    if (ok) atomicOr(&s_match[warp][d], 1u << lane);
+    __syncwarp();
+    uint32_t peers = 0u, old = 0u;
     if (ok) {
+      peers = s_match[warp][d];
       old = s_wc[warp][d];
       rank[k] = old + __popc(peers & lt);
     }
     __syncwarp();
-    if (ok && lane == __ffs(peers) - 1) s_wc[warp][d] = old + __popc(peers);
+    if (ok && (peers & lt) == 0u) {
+      s_wc[warp][d] = old + __popc(peers);
+      s_match[warp][d] = 0u;
+    }
     __syncwarp();
   }
   __syncthreads();
@@ -306,7 +304,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
   __syncthreads();
 
 #pragma unroll
-  for (int k = 0; k < kSortItems; ++k) {
+  for (int k = 0; k < ITEMS; ++k) {
     long idx = seg + k * 32 + lane;
     if (idx < n) {
       const uint32_t d = (uint32_t)((key[k] >> shift) & 0xffu);
@@ -370,29 +368,39 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
 }
 
 // Launches one sort pass with its staging buffer (dynamic shared memory).
-template <typename K, int MODE>
-static int launch_sort_pass(int tiles, cudaStream_t st, const K* kin, const uint32_t* vin,
-                            K* kout, uint32_t* vout, int n, int shift,
-                            const uint32_t* hist, uint32_t* status, uint32_t* ctr,
-                            unsigned* err, const float4* pos, float4* pos_sorted,
-                            const SimDesc* sims, int nsims, bool chained = false) {
-  const int smem = kSortTile * (int)(sizeof(K) + sizeof(uint32_t));
-  NB_CUDA(cudaFuncSetAttribute(k_sort_pass<K, MODE>,
+template <typename K, int MODE, int ITEMS>
+static int launch_sort_pass_items(int tiles, cudaStream_t st, bool chained, const K* kin,
+                                  const uint32_t* vin, K* kout, uint32_t* vout, int n, int shift,
+                                  const uint32_t* hist, uint32_t* status, uint32_t* ctr,
+                                  unsigned* err, const float4* pos, float4* pos_sorted,
+                                  const SimDesc* sims, int nsims) {
+  const int smem = kSortThreads * ITEMS * (int)(sizeof(K) + sizeof(uint32_t));
+  NB_CUDA(cudaFuncSetAttribute(k_sort_pass<K, MODE, ITEMS>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   if (chained)
-    return launch_chained(k_sort_pass<K, MODE>, tiles, kSortThreads, smem, st, kin, vin, kout,
-                          vout, n, shift, hist, status, ctr, err, pos, pos_sorted, sims,
+    return launch_chained(k_sort_pass<K, MODE, ITEMS>, tiles, kSortThreads, smem, st, kin, vin,
+                          kout, vout, n, shift, hist, status, ctr, err, pos, pos_sorted, sims,
                           nsims);
-  k_sort_pass<K, MODE><<<tiles, kSortThreads, smem, st>>>(
+  k_sort_pass<K, MODE, ITEMS><<<tiles, kSortThreads, smem, st>>>(
       kin, vin, kout, vout, n, shift, hist, status, ctr, err, pos, pos_sorted, sims, nsims);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
 
+template <typename K, int MODE, typename... Args>
+static int launch_sort_pass(cudaStream_t st, bool chained, int n, const K* kin,
+                            const uint32_t* vin, K* kout, uint32_t* vout, Args... rest) {
+  const int tiles = sort_tiles(n);
+  if (sort_items(n) == kSortSmallItems)
+    return launch_sort_pass_items<K, MODE, kSortSmallItems>(tiles, st, chained, kin, vin, kout,
+                                                            vout, n, rest...);
+  return launch_sort_pass_items<K, MODE, kSortItems>(tiles, st, chained, kin, vin, kout, vout,
+                                                     n, rest...);
+}
+
 template <typename K>
 static int sort_impl(Workspace& w, const StepArgs& a, cudaStream_t st) {
   const int passes = sort_passes(a.key_bits);
-  const int tiles = (a.n + kSortTile - 1) / kSortTile;
   K* kin = (K*)w.keys;
   K* kalt = (K*)w.keys_alt;
   // the first pass takes the particle index as its value (the keys are in
@@ -405,13 +413,13 @@ static int sort_impl(Workspace& w, const StepArgs& a, cudaStream_t st) {
     uint32_t* status = w.hist + 8 * kSortRadix + 8 + (size_t)p * w.status_tiles * kSortRadix;
     uint32_t* ctr = w.tile_ctr + p;
     if (p == passes - 1)
-      NB_TRY((launch_sort_pass<K, kSortLast>(tiles, st, kin, vin, kalt, valt, a.n, 8 * p,
-                                             hist, status, ctr, w.err, a.pos,
-                                             w.pos_sorted, nullptr, 0, true)));
+      NB_TRY((launch_sort_pass<K, kSortLast>(st, true, a.n, kin, vin, kalt, valt, 8 * p, hist,
+                                             status, ctr, w.err, (const float4*)a.pos,
+                                             w.pos_sorted, (const SimDesc*)nullptr, 0)));
     else
-      NB_TRY((launch_sort_pass<K, kSortMid>(tiles, st, kin, vin, kalt, valt, a.n, 8 * p,
-                                            hist, status, ctr, w.err, nullptr, nullptr,
-                                            nullptr, 0, true)));
+      NB_TRY((launch_sort_pass<K, kSortMid>(st, true, a.n, kin, vin, kalt, valt, 8 * p, hist,
+                                            status, ctr, w.err, (const float4*)nullptr,
+                                            (float4*)nullptr, (const SimDesc*)nullptr, 0)));
     K* tk = kin; kin = kalt; kalt = tk;
     uint32_t* tv = valt; valt = vnext; vin = tv; vnext = tv;
   }
@@ -439,10 +447,10 @@ int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st) {
 //
 // Bound: latency.  Up to about 100,000 keys a onesweep pass takes 9 us whatever
 // n is (launch, ticket, look-back); here a pass is two cluster barriers (0.5 us
-// each), and the rank (0.5 us for every 1,024 keys of a slice) and scatter of
-// n / 16 keys per SM: 20 us for the keys and four passes at n = 4,096 against
-// 42, 27 against 47 at 20,011, 45 against 51 at 65,536.  512 threads: with 1,024
-// the barriers cost more than the wider rank gains (31 us at 20,011).
+// each), and the rank and scatter of n / 16 keys per SM: 19 us for the keys and
+// four passes at n = 4,096 against 42, 25 against 47 at 20,011, 39 against 41 at
+// 65,536.  512 threads: with 1,024 the barriers cost more than the wider rank
+// gains.
 // ---------------------------------------------------------------------------
 constexpr int kClusterCtas = 16;
 constexpr int kClusterThreads = 512;
@@ -452,10 +460,39 @@ constexpr int kClusterItems = 8;
 constexpr int kClusterSlice = kClusterThreads * kClusterItems;   // keys per CTA at most
 constexpr int kClusterMax = kClusterCtas * kClusterSlice;
 
-__host__ __device__ constexpr size_t cluster_sort_smem(size_t key_bytes, int slice) {
-  // keys and values twice, digit counts by warp, by part of the warps and by
-  // CTA (twice), two words per digit, and scan words
-  return 2 * (size_t)slice * (key_bytes + 4) + kClusterWarps * kSortRadix * 2 +
+// A slice of keys and values in shared memory.  32-bit keys lie beside their
+// value, one 8-byte store to another CTA's slice (45 -> 39 us at 65,536
+// particles against two arrays); 64-bit ones in an array of their own (16-byte
+// entries take 118 us at 49,152, two arrays 74).
+template <typename K>
+struct Slice {
+  K* key;
+  uint32_t* val;
+  __device__ Slice(void* raw, int slice, int which)
+      : key((K*)raw + which * slice), val((uint32_t*)((K*)raw + 2 * slice) + which * slice) {}
+  __device__ Slice(const Slice& s, cg::cluster_group& c, int r)
+      : key(c.map_shared_rank(s.key, r)), val(c.map_shared_rank(s.val, r)) {}
+  __device__ void get(int i, K& k, uint32_t& v) const { k = key[i]; v = val[i]; }
+  __device__ void put(uint32_t i, K k, uint32_t v) const { key[i] = k; val[i] = v; }
+};
+template <>
+struct Slice<uint32_t> {
+  uint2* kv;
+  __device__ Slice(void* raw, int slice, int which) : kv((uint2*)raw + which * slice) {}
+  __device__ Slice(const Slice& s, cg::cluster_group& c, int r) : kv(c.map_shared_rank(s.kv, r)) {}
+  __device__ void get(int i, uint32_t& k, uint32_t& v) const {
+    const uint2 e = kv[i];
+    k = e.x;
+    v = e.y;
+  }
+  __device__ void put(uint32_t i, uint32_t k, uint32_t v) const { kv[i] = make_uint2(k, v); }
+};
+
+template <typename K>
+__host__ __device__ constexpr size_t cluster_sort_smem(int slice) {
+  // keys and values twice, lane masks and digit counts by warp, counts by part
+  // of the warps and by CTA (twice), two words per digit, and scan words
+  return 2 * (size_t)slice * (sizeof(K) + 4) + kClusterWarps * kSortRadix * (4 + 2) +
          kClusterParts * kSortRadix * 4 + (2 * kClusterCtas + 2) * kSortRadix * 4 + 16 * 4;
 }
 
@@ -466,9 +503,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                    float4* __restrict__ pos_sorted, int slice, uint32_t slice_inv, int passes,
                    unsigned* err) {
   extern __shared__ __align__(16) unsigned char s_raw[];
-  K* s_key = reinterpret_cast<K*>(s_raw);                               // [2][slice]
-  uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + 2 * slice);     // [2][slice]
-  uint16_t* s_wc = reinterpret_cast<uint16_t*>(s_val + 2 * slice);      // [warps][radix]
+  // two slices first
+  uint32_t* s_match = reinterpret_cast<uint32_t*>(s_raw + 2 * slice * (sizeof(K) + 4));   // [warps][radix]
+  uint16_t* s_wc = reinterpret_cast<uint16_t*>(s_match + kClusterWarps * kSortRadix);   // [warps][radix]
   uint32_t* s_part = reinterpret_cast<uint32_t*>(s_wc + kClusterWarps * kSortRadix);   // [parts][radix]
   uint32_t* s_cnt = s_part + kClusterParts * kSortRadix;     // [2][CTAs][radix] digit counts
   uint32_t* s_tex = s_cnt + 2 * kClusterCtas * kSortRadix;      // digit's first place in the slice
@@ -482,6 +519,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   const int count = max(0, min(slice, n - first));
   const int items = (slice + kClusterThreads - 1) / kClusterThreads;
   const int seg = warp * items * 32 + lane;
+  for (int i = tid; i < kClusterWarps * kSortRadix; i += kClusterThreads) s_match[i] = 0u;
   cluster.barrier_arrive();   // waited for before the first remote store: every CTA has started
   chain_release();
   chain_wait();
@@ -505,10 +543,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   }
   for (int ps = 0; ps < passes; ++ps) {
     const int shift = 8 * ps;
-    K* ck = s_key + (ps & 1) * slice;             // this pass's slice, then its staging
-    uint32_t* cv = s_val + (ps & 1) * slice;
-    K* nk = s_key + ((ps + 1) & 1) * slice;       // the next pass's slice
-    uint32_t* nv = s_val + ((ps + 1) & 1) * slice;
+    const Slice<K> cur(s_raw, slice, ps & 1);          // this pass's slice, then its staging
+    const Slice<K> next(s_raw, slice, (ps + 1) & 1);   // the next pass's slice
     uint32_t* cnt = s_cnt + (ps & 1) * kClusterCtas * kSortRadix;
     reinterpret_cast<uint4*>(s_wc)[tid] = make_uint4(0u, 0u, 0u, 0u);
     if (ps > 0) {
@@ -516,27 +552,34 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       for (int k = 0; k < kClusterItems; ++k) {
         const int i = seg + 32 * k;
         if (k < items && i < count) {
-          key[k] = ck[i];
-          val[k] = cv[i];
+          cur.get(i, key[k], val[k]);
         }
       }
     }
     __syncthreads();
     uint32_t rank[kClusterItems];
     uint16_t* wc = s_wc + warp * kSortRadix;
+    uint32_t* match = s_match + warp * kSortRadix;
 #pragma unroll
     for (int k = 0; k < kClusterItems; ++k) {
       if (k >= items) break;
       const bool ok = seg + 32 * k < count;
       const uint32_t d = ok ? (uint32_t)((key[k] >> shift) & 0xffu) : 0u;
-      const uint32_t peers = digit_peers(d, ok);
-      uint32_t old = 0;
+      // the lanes with this digit set their bits in its word; the first of
+      // them counts them and clears it
+      if (ok) atomicOr(&match[d], 1u << lane);
+      __syncwarp();
+      uint32_t peers = 0u, old = 0u;
       if (ok) {
+        peers = match[d];
         old = wc[d];
         rank[k] = old + __popc(peers & lt);
       }
       __syncwarp();
-      if (ok && lane == __ffs(peers) - 1) wc[d] = (uint16_t)(old + __popc(peers));
+      if (ok && (peers & lt) == 0u) {
+        wc[d] = (uint16_t)(old + __popc(peers));
+        match[d] = 0u;
+      }
       __syncwarp();
     }
     __syncthreads();
@@ -612,8 +655,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         const uint32_t dg = (uint32_t)((key[k] >> shift) & 0xffu);
         const uint32_t at = s_tex[dg] + wc[dg] + rank[k];
         if (at < (uint32_t)count) {
-          ck[at] = key[k];
-          cv[at] = val[k];
+          cur.put(at, key[k], val[k]);
         } else {
           raise_err(err, NB_DEVERR_SORT);
         }
@@ -625,8 +667,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     for (int k = 0; k < kClusterItems; ++k) {
       const int i = tid + k * kClusterThreads;
       if (i >= count) break;
-      const K kk = ck[i];
-      const uint32_t vv = cv[i];
+      K kk;
+      uint32_t vv;
+      cur.get(i, kk, vv);
       const uint32_t p = s_base[(uint32_t)((kk >> shift) & 0xffu)] + (uint32_t)i;
       if (p >= (uint32_t)n || vv >= (uint32_t)n) {
         raise_err(err, NB_DEVERR_SORT);
@@ -638,8 +681,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         pos_sorted[p] = pos[vv];
       } else {
         const uint32_t r = __umulhi(p, slice_inv);   // p / slice
-        cluster.map_shared_rank(nk, r)[p - r * slice] = kk;
-        cluster.map_shared_rank(nv, r)[p - r * slice] = vv;
+        Slice<K>(next, cluster, r).put(p - r * slice, kk, vv);
       }
     }
     if (!last) cluster.sync();   // the next slice is complete
@@ -651,7 +693,7 @@ static int cluster_sort_config(int slice, cudaLaunchConfig_t* cfg, cudaLaunchAtt
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = kClusterCtas;
   cfg->blockDim = kClusterThreads;
-  cfg->dynamicSmemBytes = cluster_sort_smem(sizeof(K), slice);
+  cfg->dynamicSmemBytes = cluster_sort_smem<K>(slice);
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = kClusterCtas;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -660,7 +702,7 @@ static int cluster_sort_config(int slice, cudaLaunchConfig_t* cfg, cudaLaunchAtt
   NB_CUDA(cudaFuncSetAttribute(k_sort_cluster<K>, cudaFuncAttributeNonPortableClusterSizeAllowed,
                                1));
   NB_CUDA(cudaFuncSetAttribute(k_sort_cluster<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)cluster_sort_smem(sizeof(K), kClusterSlice)));
+                               (int)cluster_sort_smem<K>(kClusterSlice)));
   return NB_OK;
 }
 
@@ -690,12 +732,12 @@ static bool cluster_sort_fits() {
   return known[dev] == 1;
 }
 
-// Step of a simulation, one launch against Morton kernel and onesweep passes:
-// 30 bits 52 against 66 us at n = 1,000, 115 / 136 at 20,011, 161 / 164 at 65,536;
-// 63 bits 134 / 168 at 20,011, 181 / 197 at 50,000, equal near 65,536 (8 passes
-// over n / 16 keys per SM, while the onesweep's grow little with n).
+// Keys and sort, one launch against Morton kernel and onesweep passes: 30 bits
+// 24 / 34 us at n = 10,000, 34 / 40 at 40,000, equal at 65,536; 63 bits 42 / 60 at
+// 10,000, 58 / 65 at 30,000, equal at 40,000 (8 passes over n / 16 keys per SM, while
+// the onesweep's grow little with n).
 bool sort_in_cluster(int n, int key_bits) {
-  if (n > (key_bits == 63 ? kClusterMax * 3 / 4 : kClusterMax)) return false;
+  if (n > (key_bits == 63 ? kClusterMax / 16 * 9 : kClusterMax)) return false;
   return key_bits == 63 ? cluster_sort_fits<uint64_t>() : cluster_sort_fits<uint32_t>();
 }
 
@@ -1453,7 +1495,6 @@ int ens_sort_passes() { return (kEnsKeyBits + 7) / 8; }
 
 int launch_ens_sort(EnsArgs& e, cudaStream_t st) {
   const int passes = ens_sort_passes();
-  const int tiles = (e.nslots + kSortTile - 1) / kSortTile;
   uint64_t* kin = e.keys;
   uint64_t* kalt = e.keys_alt;
   uint32_t* vin = e.perm;
@@ -1464,12 +1505,12 @@ int launch_ens_sort(EnsArgs& e, cudaStream_t st) {
     uint32_t* ctr = e.tile_ctr + p;
     if (p == passes - 1)
       NB_TRY((launch_sort_pass<uint64_t, kSortLastEnsemble>(
-          tiles, st, kin, vin, kalt, valt, e.nslots, 8 * p, hist, status, ctr, e.err,
-          e.pos, e.pos_sorted, e.sims, e.nsims)));
+          st, false, e.nslots, kin, vin, kalt, valt, 8 * p, hist, status, ctr, e.err,
+          (const float4*)e.pos, e.pos_sorted, e.sims, e.nsims)));
     else
       NB_TRY((launch_sort_pass<uint64_t, kSortMid>(
-          tiles, st, kin, vin, kalt, valt, e.nslots, 8 * p, hist, status, ctr, e.err,
-          nullptr, nullptr, nullptr, 0)));
+          st, false, e.nslots, kin, vin, kalt, valt, 8 * p, hist, status, ctr, e.err,
+          (const float4*)nullptr, (float4*)nullptr, (const SimDesc*)nullptr, 0)));
     uint64_t* tk = kin; kin = kalt; kalt = tk;
     uint32_t* tv = vin; vin = valt; valt = tv;
   }
@@ -1577,9 +1618,16 @@ int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st) 
 int warm_lbvh_kernels() {
   return warm_fns(k_morton<uint32_t>, k_morton<uint64_t>, k_ens_morton,
                   k_sort_cluster<uint32_t>, k_sort_cluster<uint64_t>,
-                  k_sort_pass<uint32_t, kSortMid>, k_sort_pass<uint32_t, kSortLast>,
-                  k_sort_pass<uint64_t, kSortMid>, k_sort_pass<uint64_t, kSortLast>,
-                  k_sort_pass<uint64_t, kSortLastEnsemble>, k_build_level<uint32_t, 256, 256>,
+                  k_sort_pass<uint32_t, kSortMid, kSortItems>,
+                  k_sort_pass<uint32_t, kSortLast, kSortItems>,
+                  k_sort_pass<uint64_t, kSortMid, kSortItems>,
+                  k_sort_pass<uint64_t, kSortLast, kSortItems>,
+                  k_sort_pass<uint64_t, kSortLastEnsemble, kSortItems>,
+                  k_sort_pass<uint32_t, kSortMid, kSortSmallItems>,
+                  k_sort_pass<uint32_t, kSortLast, kSortSmallItems>,
+                  k_sort_pass<uint64_t, kSortMid, kSortSmallItems>,
+                  k_sort_pass<uint64_t, kSortLast, kSortSmallItems>,
+                  k_sort_pass<uint64_t, kSortLastEnsemble, kSortSmallItems>, k_build_level<uint32_t, 256, 256>,
                   k_build_level<uint32_t, 256, 128>, k_build_level<uint32_t, 512, 512>,
                   k_build_level<uint32_t, 512, 256>, k_build_level<uint32_t, 1024, 512>,
                   k_build_level<uint64_t, 256, 256>, k_build_level<uint64_t, 256, 128>,

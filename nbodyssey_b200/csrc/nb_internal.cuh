@@ -69,15 +69,29 @@ struct __align__(16) PairRec {
 constexpr int kStack = 128;
 
 // Onesweep sort geometry.
-// 512 threads (the first 256 own one digit each in the per-digit steps),
-// 8 keys per thread, 2 CTAs per SM: at 1M keys a pass is one wave of 245
-// tiles.  A tile's latency and the look-back's prefix propagation through
-// the tiles, not bandwidth, set the pass time; this geometry measured best
-// against 256 threads with 4096 or 2048 keys and 1024 keys per tile.
+// 512 threads (the first 256 own one digit each in the per-digit steps), 2 CTAs
+// per SM.  A tile's latency and the look-back's prefix propagation through the
+// tiles, not bandwidth, set the pass time.  8 keys per thread: at 1M keys a pass
+// is one wave of 245 tiles (256 threads with 4096 or 2048 keys and 1024 keys per
+// tile measured slower).  Up to kSortSmallMax keys, where half the tile still
+// gives no more tiles than SMs, 4 keys per thread: the rank takes half as long
+// (keys and four passes 42 against 49 us at n = 100,000, 49 / 52 at 300,000, and 94
+// against 79 at 1M; 2 keys per thread 41 and 54).
 constexpr int kSortThreads = 512;
 constexpr int kSortItems = 8;
+constexpr int kSortSmallItems = 4;
 constexpr int kSortCtasPerSm = 2;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per tile
+constexpr int kSortSmallMax = 148 * kSortThreads * kSortSmallItems;
+inline int sort_items(int n) { return n <= kSortSmallMax ? kSortSmallItems : kSortItems; }
+inline int sort_tiles(int n) {
+  const int tile = kSortThreads * sort_items(n);
+  return (n + tile - 1) / tile;
+}
+// tiles of look-back words that serve every size up to cap
+inline int sort_status_tiles(int cap) {
+  const int small = sort_tiles(cap < kSortSmallMax ? cap : kSortSmallMax), all = sort_tiles(cap);
+  return small > all ? small : all;
+}
 constexpr int kSortRadix = 256;
 
 // All-pairs source layout: particles are packed in pairs as two float4,

@@ -418,7 +418,7 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
   e.nslots = extent;
   e.nblocks = extent / 32;
   // look-back words laid out (and cleared) for this step's extent only
-  e.status_tiles = (extent + kSortTile - 1) / kSortTile;
+  e.status_tiles = sort_tiles(extent);
   e.kick_drift = true;
   e.kick_after = true;
   NB_TRY(launch_ens_prep(e, s->stream));
@@ -556,7 +556,7 @@ int nb_server_create(size_t hbm_budget_bytes, int max_sims, nb_server** out) {
     if ((rc = srv_alloc(s, &e.box_hi, S)) != NB_OK) break;
     if ((rc = srv_alloc(s, &e.bbox_min, 4 * (size_t)max_sims)) != NB_OK) break;
     if ((rc = srv_alloc(s, &e.bbox_max, 4 * (size_t)max_sims)) != NB_OK) break;
-    e.status_tiles = (int)((S + kSortTile - 1) / kSortTile);
+    e.status_tiles = sort_status_tiles((int)S);
     const size_t words = 8 * kSortRadix + 8 + (size_t)8 * e.status_tiles * kSortRadix;
     if ((rc = srv_alloc(s, &e.hist, words)) != NB_OK) break;
     e.tile_ctr = e.hist + 8 * kSortRadix;

@@ -1,7 +1,7 @@
 """The two sorts of the tree build against the oracle's stable sort: one
-cluster launch (up to 65,536 particles, 49,152 with 63-bit keys; slices of
+cluster launch (up to 65,536 particles, 36,864 with 63-bit keys; slices of
 n / 16 rounded up to 32 keys, 512 threads) and the onesweep passes above
-(4,096-key tiles)."""
+(2,048-key tiles up to 303,104 keys, then 4,096)."""
 import numpy as np
 import pytest
 
@@ -22,8 +22,9 @@ def _check(pos, bits):
 
 
 @pytest.mark.parametrize("n", [2, 32, 33, 511, 512, 513, 16 * 512 - 1, 16 * 512, 16 * 512 + 1,
-                               20_011, 49_151, 49_152, 49_153, 53_248, 53_249,
-                               65_535, 65_536, 65_537, 69_632, 69_633])
+                               20_011, 36_863, 36_864, 36_865, 53_248, 53_249,
+                               65_535, 65_536, 65_537, 69_632, 69_633, 303_104, 303_105,
+                               307_201])
 @pytest.mark.parametrize("bits", [30, 63])
 def test_sizes(n, bits):
     pos, _ = ic.two_disks(n, seed=n)
