@@ -140,7 +140,7 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   NB_TRY(dalloc(&w.parent, 2 * (size_t)cap));
   for (int i = 0; i < 2; ++i) {
     NB_TRY(dalloc(&w.seg[i], build_seg_entries(cap)));
-    NB_TRY(dalloc(&w.seg_count[i], build_seg_entries(cap)));
+    NB_TRY(dalloc(&w.seg_count[i], build_groups(cap)));
   }
   NB_TRY(dalloc(&w.sums, ni));
   NB_TRY(dalloc(&w.box_lo, ni));

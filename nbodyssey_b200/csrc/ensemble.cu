@@ -256,7 +256,7 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
       const size_t segs = plan_seg_entries(b, nsims);
       for (int i = 0; i < 2; ++i) {
         if ((rc = ens_alloc(h, &e.seg[i], segs)) != NB_OK) break;
-        if ((rc = ens_alloc(h, &e.seg_count[i], segs)) != NB_OK) break;
+        if ((rc = ens_alloc(h, &e.seg_count[i], plan_groups(b, nsims))) != NB_OK) break;
       }
       if (rc != NB_OK) break;
     }

@@ -828,11 +828,11 @@ struct LevelArgs {
   float4* box_lo;
   float4* box_hi;
   const int2* in_seg;               // later levels: (position, delta) lists
-  const int* in_count;
+  const int2* in_count;             // per list its length and last delta
   int in_groups;                    // CTAs of the level below
   long long in_span;                // leaves per CTA of the level below
   int2* out_seg;                    // nullptr at the last level
-  int* out_count;
+  int2* out_count;
   int seg;                          // segment capacity
   int fan;                          // segments per CTA
   unsigned* err;
@@ -1155,36 +1155,33 @@ __global__ void __launch_bounds__(T, G ? 1024 / T : 1) k_build_level(LevelArgs a
     }
     if (tid == 0) sm.delta[0] = run.A > 0 ? split_delta(keys, run.A - 1) : kDeltaFirst;
   } else {
-    const int r0 = sfirst, r1 = sfirst + scount;
-    if (warp == 0) {   // segment offsets (fan <= 32)
-      const int c = r0 + lane < r1 ? min(p.in_count[r0 + lane], p.seg) : 0;
-      int incl = c;
+    // every warp reads all segments' counts and one segment's entries, all at
+    // once (those past its count are dropped): one trip to L2
+    static_assert(FIRST || level_fan(30) <= T / 32, "one warp per segment");
+    constexpr int kPer = level_seg(63) / 32;
+    const int cl = lane < scount ? min(p.in_count[sfirst + lane].x, p.seg) : 0;
+    int2 v[kPer];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      sm.scan[lane] = incl - c;
-      if (lane == 31) sm.scan[32] = incl;
-      if (lane == 0) {   // the last entry below is the split left of this run
-        int d = kDeltaFirst;
-        if (g > 0) {
-          const int cp = min(p.in_count[r0 - 1], p.seg);
-          if (cp > 0) d = p.in_seg[(size_t)(r0 - 1) * p.seg + cp - 1].y;
-        }
-        sm.delta[0] = d;
-      }
+    for (int i = 0; i < kPer; ++i)
+      if (warp < scount && lane + 32 * i < p.seg)
+        v[i] = p.in_seg[(size_t)(sfirst + warp) * p.seg + lane + 32 * i];
+    // the last split of the segment before: left of this run
+    if (tid == 0) sm.delta[0] = g > 0 ? p.in_count[sfirst - 1].y : kDeltaFirst;
+    int incl = cl;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
     }
-    __syncthreads();
-    run.M = sm.scan[32];
-    // one warp per segment
-    for (int r = r0 + warp; r < r1; r += T / 32) {
-      const int off = sm.scan[r - r0];
-      const int c = sm.scan[r - r0 + 1] - off;
-      for (int e = lane; e < c; e += 32) {
-        const int2 v = p.in_seg[(size_t)r * p.seg + e];
-        sm.pos[off + e] = v.x;
-        sm.delta[off + e + 1] = v.y;
+    run.M = __shfl_sync(0xffffffffu, incl, 31);
+    const int off = __shfl_sync(0xffffffffu, incl - cl, warp);
+    const int c = __shfl_sync(0xffffffffu, cl, warp);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int e = lane + 32 * i;
+      if (warp < scount && e < c) {
+        sm.pos[off + e] = v[i].x;
+        sm.delta[off + e + 1] = v[i].y;
       }
     }
     // region index of segment r within the tree: g * fan + (r - sfirst)
@@ -1326,7 +1323,7 @@ __global__ void __launch_bounds__(T, G ? 1024 / T : 1) k_build_level(LevelArgs a
     }
   }
   if (tid == 0) {
-    p.out_count[blockIdx.x] = min(total, p.seg);
+    p.out_count[blockIdx.x] = make_int2(min(total, p.seg), sm.delta[run.M]);
     if (total > p.seg) raise_err(a.err(), NB_DEVERR_TREE);
   }
 }
@@ -1367,8 +1364,10 @@ static int leaf_group(int n, int fan) {
   return 1024;
 }
 
+size_t build_groups(int cap) { return (size_t)cap / 256 + 1; }   // the smallest groups
+
 size_t build_seg_entries(int cap) {
-  return ((size_t)cap / 256 + 1) * level_seg(63);   // the smallest groups
+  return build_groups(cap) * level_seg(63);
 }
 
 template <typename K>
@@ -1571,8 +1570,12 @@ int plan_build(const SimDesc* sims, int nsims, BuildPlan& plan) {
   return NB_OK;
 }
 
+size_t plan_groups(int slots, int nsims) {
+  return (size_t)slots / kEnsLeafGroup + (size_t)nsims + 1;
+}
+
 size_t plan_seg_entries(int slots, int nsims) {
-  return ((size_t)slots / kEnsLeafGroup + (size_t)nsims + 1) * level_seg(30);
+  return plan_groups(slots, nsims) * level_seg(30);
 }
 
 int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st) {

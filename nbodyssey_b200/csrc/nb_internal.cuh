@@ -116,7 +116,7 @@ struct Workspace {
   PairRec* pairs = nullptr;       // [cap] child pairs by split + the root's
   int* parent = nullptr;          // [2cap-1]
   int2* seg[2] = {nullptr, nullptr};      // open splits per build CTA,
-  int* seg_count[2] = {nullptr, nullptr}; // ping-pong between levels
+  int2* seg_count[2] = {nullptr, nullptr}; // ping-pong between levels
   double4* sums = nullptr;        // [cap-1] FP64 mass-weighted sums
   float4* box_lo = nullptr;       // [cap-1]
   float4* box_hi = nullptr;       // [cap-1]
@@ -198,6 +198,7 @@ int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st);
 // memory (on a device that can hold it); the sort scratch is not used
 bool sort_in_cluster(int n, int key_bits);
 int launch_sort_cluster(Workspace& w, const StepArgs& a, cudaStream_t st);
+size_t build_groups(int cap);       // first-level CTAs at most, for any n <= cap
 size_t build_seg_entries(int cap);
 int launch_build(Workspace& w, const StepArgs& a, cudaStream_t st);
 int launch_com(Workspace& w, const StepArgs& a, cudaStream_t st);
@@ -465,7 +466,7 @@ struct EnsArgs {
   bool kick_after;
   const BuildRun* runs;       // tree-build plan (all levels)
   int2* seg[2];               // open splits between build levels
-  int* seg_count[2];
+  int2* seg_count[2];
   // the Barnes-Hut walk's work queue: per semantics (0 warp, 1 thread) the
   // 32-slot blocks to walk, costliest first, and a counter each (zeroed by
   // the launcher every step)
@@ -565,6 +566,7 @@ int launch_ens_sort(EnsArgs& e, cudaStream_t st);   // updates e.keys / e.perm
 // Tree build of all simulations (k_lbvh.cu): a host plan of level runs,
 // uploaded to e.runs, then one launch per level.
 int plan_build(const SimDesc* sims, int nsims, BuildPlan& plan);
+size_t plan_groups(int slots, int nsims);
 size_t plan_seg_entries(int slots, int nsims);
 int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st);
 int launch_walk_pair_ens(const EnsArgs& e, cudaStream_t st);

@@ -574,7 +574,7 @@ int nb_server_create(size_t hbm_budget_bytes, int max_sims, nb_server** out) {
       const size_t segs = plan_seg_entries((int)S, max_sims);
       for (int i = 0; i < 2; ++i) {
         if ((rc = srv_alloc(s, &e.seg[i], segs)) != NB_OK) break;
-        if ((rc = srv_alloc(s, &e.seg_count[i], segs)) != NB_OK) break;
+        if ((rc = srv_alloc(s, &e.seg_count[i], plan_groups((int)S, max_sims))) != NB_OK) break;
       }
       if (rc != NB_OK) break;
     }
