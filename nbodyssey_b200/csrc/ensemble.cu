@@ -13,6 +13,48 @@
 
 #include "nb_internal.cuh"
 
+namespace nb {
+
+int EnsFork::create() {
+  NB_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&start, &walks, &done})
+    NB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  return NB_OK;
+}
+
+void EnsFork::destroy() {
+  if (aux) {
+    cudaStreamSynchronize(aux);
+    cudaStreamDestroy(aux);
+  }
+  for (cudaEvent_t e : {start, walks, done})
+    if (e) cudaEventDestroy(e);
+  *this = EnsFork{};
+}
+
+int launch_ens_step(EnsArgs& e, const BuildPlan& plan, const EnsAllPairs& ap, bool any_tree,
+                    const EnsFork& fork, cudaStream_t st) {
+  NB_TRY(launch_ens_prep(e, st));
+  if (!any_tree) return launch_ens_allpairs(e, ap, st);
+  const bool beside = !ap.args.empty() || !ap.sym.args.empty();
+  if (beside) {
+    NB_CUDA(cudaEventRecord(fork.start, st));
+    NB_CUDA(cudaStreamWaitEvent(fork.aux, fork.start, 0));
+    NB_TRY(launch_ens_allpairs(e, ap, fork.aux));
+  }
+  NB_TRY(launch_ens_morton(e, st));
+  NB_TRY(launch_ens_sort(e, st));
+  NB_TRY(launch_ens_levels(e, plan, st));
+  NB_TRY(launch_walk_pair_ens(e, fork, st));
+  if (beside || (e.walk_nitems[0] > 0 && e.walk_nitems[1] > 0)) {
+    NB_CUDA(cudaEventRecord(fork.done, fork.aux));
+    NB_CUDA(cudaStreamWaitEvent(st, fork.done, 0));
+  }
+  return NB_OK;
+}
+
+}  // namespace nb
+
 using namespace nb;
 
 struct nb_ensemble {
@@ -21,6 +63,7 @@ struct nb_ensemble {
   std::vector<int> n, base;
   std::vector<nb_params> params;
   cudaStream_t stream = nullptr;
+  EnsFork fork;
   EnsArgs e{};                 // device pointers as allocated
   SimDesc* d_sims = nullptr;
   int* d_blk = nullptr;
@@ -58,6 +101,7 @@ int ens_alloc(nb_ensemble* h, T** p, size_t count) {
 void ens_free(nb_ensemble* h) {
   if (!h) return;
   if (h->stream) cudaStreamSynchronize(h->stream);
+  h->fork.destroy();
   if (h->graph) cudaGraphExecDestroy(h->graph);
   for (auto& ev : h->slots)
     if (ev) cudaEventDestroy(ev);
@@ -89,16 +133,7 @@ int ens_enqueue(nb_ensemble* h, bool prime) {
   EnsArgs e = h->e;
   e.kick_drift = !prime;
   e.kick_after = !prime;
-  cudaStream_t st = h->stream;
-  NB_TRY(launch_ens_prep(e, st));
-  if (h->any_tree) {
-    NB_TRY(launch_ens_morton(e, st));
-    NB_TRY(launch_ens_sort(e, st));
-    NB_TRY(launch_ens_levels(e, h->plan, st));
-    NB_TRY(launch_walk_pair_ens(e, st));
-  }
-  NB_TRY(launch_ens_allpairs(e, h->ap, st));
-  return NB_OK;
+  return launch_ens_step(e, h->plan, h->ap, h->any_tree, h->fork, h->stream);
 }
 
 int ens_capture(nb_ensemble* h) {
@@ -264,6 +299,7 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     cudaError_t ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaMallocHost((void**)&h->h_err, sizeof(unsigned));
     if (ce != cudaSuccess) { rc = set_error(NB_ERR_CUDA, cudaGetErrorString(ce)); break; }
+    if ((rc = h->fork.create()) != NB_OK) break;
     cudaStream_t st = h->stream;
     // defined contents everywhere: zero state in the gaps, in-range indices
     ce = cudaMemsetAsync(e.pos, 0, S * 16, st);

@@ -626,17 +626,24 @@ void plan_walk_queue(const SimDesc* sims, int nsims, std::vector<int> items[2]) 
   }
 }
 
-int launch_walk_pair_ens(const EnsArgs& e, cudaStream_t st) {
+// Thread semantics' walk, the longer one, goes to the fork's stream when there
+// are both; the caller joins it.
+int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st) {
   NB_CUDA(cudaMemsetAsync(e.walk_ctr, 0, 2 * sizeof(int), st));
   const int cap = device_sm_count() * 8;   // 8 resident blocks of 4 warps per SM
-  for (int q = 0; q < 2; ++q) {
+  const bool both = e.walk_nitems[0] > 0 && e.walk_nitems[1] > 0;
+  if (both) {
+    NB_CUDA(cudaEventRecord(fork.walks, st));
+    NB_CUDA(cudaStreamWaitEvent(fork.aux, fork.walks, 0));
+  }
+  for (int q = 1; q >= 0; --q) {
     const int n = e.walk_nitems[q];
     if (n <= 0) continue;
     const int blocks = std::min((n + kEnsW - 1) / kEnsW, cap);
     if (q == 0) k_walk_pair_ens<false><<<blocks, kEnsW * 32, 0, st>>>(e);
-    else k_walk_pair_ens<true><<<blocks, kEnsW * 32, 0, st>>>(e);
+    else k_walk_pair_ens<true><<<blocks, kEnsW * 32, 0, both ? fork.aux : st>>>(e);
+    NB_CUDA(cudaGetLastError());
   }
-  NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
 

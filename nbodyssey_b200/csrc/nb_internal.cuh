@@ -569,7 +569,23 @@ int plan_build(const SimDesc* sims, int nsims, BuildPlan& plan);
 size_t plan_groups(int slots, int nsims);
 size_t plan_seg_entries(int slots, int nsims);
 int launch_ens_levels(const EnsArgs& e, const BuildPlan& plan, cudaStream_t st);
-int launch_walk_pair_ens(const EnsArgs& e, cudaStream_t st);
+// A second stream beside a batch's own and the events between them.  A step
+// forks to it what does not depend on the other simulations' work and joins it
+// before it ends, so that nothing outside sees it: the all-pairs simulations
+// run beside the tree pipeline, whose sort and build leave most of the device
+// idle, and the two semantics' walks one beside the other, so that the last long
+// walks of one do not leave the SMs to themselves.
+struct EnsFork {
+  cudaStream_t aux = nullptr;
+  cudaEvent_t start = nullptr, walks = nullptr, done = nullptr;
+  int create();
+  void destroy();
+};
+// All kernels of one step (or of a(x) alone) of a batch after its plans are on
+// the device.
+int launch_ens_step(EnsArgs& e, const BuildPlan& plan, const EnsAllPairs& ap, bool any_tree,
+                    const EnsFork& fork, cudaStream_t st);
+int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st);
 // Host: the walk queue of a simulation table (the Barnes-Hut simulations'
 // 32-slot blocks per semantics, costliest simulation first: larger n and
 // smaller theta walk longer); items[0] / items[1] get the warp / thread

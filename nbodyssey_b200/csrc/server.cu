@@ -110,6 +110,7 @@ struct nb_server {
   BuildPlan plan;                    // tree-build levels of the running sims
   size_t plan_cap = 0;               // BuildRun entries allocated at e.runs
   cudaStream_t stream = nullptr, side = nullptr;
+  EnsFork fork;
   cudaEvent_t step_ev[kInFlight] = {};
   long long step_count = 0;
   // frames
@@ -421,14 +422,7 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
   e.status_tiles = sort_tiles(extent);
   e.kick_drift = true;
   e.kick_after = true;
-  NB_TRY(launch_ens_prep(e, s->stream));
-  if (s->any_tree) {
-    NB_TRY(launch_ens_morton(e, s->stream));
-    NB_TRY(launch_ens_sort(e, s->stream));
-    NB_TRY(launch_ens_levels(e, s->plan, s->stream));
-    NB_TRY(launch_walk_pair_ens(e, s->stream));
-  }
-  NB_TRY(launch_ens_allpairs(e, s->ap, s->stream));
+  NB_TRY(launch_ens_step(e, s->plan, s->ap, s->any_tree, s->fork, s->stream));
   NB_CUDA(cudaEventRecord(ev, s->stream));
   s->step_count += 1;
   if (s->busy_first == 0) s->busy_first = now_s();
@@ -584,6 +578,7 @@ int nb_server_create(size_t hbm_budget_bytes, int max_sims, nb_server** out) {
     if (ce != cudaSuccess) { s->h_frame = nullptr; rc = set_error(NB_ERR_NOMEM, "pinned frame ring"); break; }
     ce = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
+    if (ce == cudaSuccess && (rc = s->fork.create()) != NB_OK) break;
     for (int k = 0; k < kInFlight && ce == cudaSuccess; ++k)
       ce = cudaEventCreateWithFlags(&s->step_ev[k], cudaEventDisableTiming);
     for (int k = 0; k < kFrameSlots && ce == cudaSuccess; ++k) {
@@ -601,6 +596,7 @@ int nb_server_create(size_t hbm_budget_bytes, int max_sims, nb_server** out) {
   } while (0);
   if (rc != NB_OK) {
     std::string keep = last_error();
+    s->fork.destroy();
     for (void* p : s->dallocs) cudaFree(p);
     if (s->h_frame) cudaFreeHost(s->h_frame);
     delete s;
@@ -650,6 +646,7 @@ int nb_server_destroy(nb_server* s) {
     cudaEventDestroy(s->frame_copied[k]);
   }
   for (void* p : s->dallocs) cudaFree(p);
+  s->fork.destroy();
   if (s->ap.d_items) cudaFree(s->ap.d_items);
   if (s->ap.sym.d_table) cudaFree(s->ap.sym.d_table);
   if (s->ap.d_small) cudaFree(s->ap.d_small);
