@@ -555,10 +555,10 @@ int launch_ens_allpairs(const EnsArgs& e, const EnsAllPairs& ap, cudaStream_t st
 // momentum are reduced in FP64 in a fixed order (block partials, then the last
 // block).
 //
-// Bound: 8 packed FP32 operations and 2 MUFU rsqrt per two pairs, which fill
-// the FMA pipe (64 packed lanes a cycle and SM) and the MUFU unit (16) alike:
-// 1.09 ms for the 5e9 pairs of n = 100,000 on 148 SMs at 1.93 GHz.  Measured
-// 1.40 ms a call there; the form that took every pair in both orders with
+// Bound: 7 packed FP32 operations, 2 scalar ones and 2 MUFU rsqrt per two pairs,
+// which fill the FMA pipe (64 packed lanes a cycle and SM) and the MUFU unit (16)
+// alike: 1.09 ms for the 5e9 pairs of n = 100,000 on 148 SMs at 1.93 GHz.  Measured
+// 1.43 ms a call there; the form that took every pair in both orders with
 // scalar FP32, 3.93 ms.
 // ---------------------------------------------------------------------------
 constexpr int kEThreads = 128;
@@ -598,9 +598,9 @@ __global__ void __launch_bounds__(kEThreads) k_energy_pairs(
       q[0] = p.x; q[2] = p.y; q[4] = p.z; q[6] = p.w;
     }
     __syncthreads();
-    f2 acc[K];
+    float acc[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0ull;
+    for (int k = 0; k < K; ++k) acc[k] = 0.f;
     const int pairs = (je - jt + 1) >> 1;
     const ulonglong2* src = reinterpret_cast<const ulonglong2*>(s_src);
 #pragma unroll 4
@@ -614,15 +614,18 @@ __global__ void __launch_bounds__(kEThreads) k_energy_pairs(
         const f2 r2 = add2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), e2);
         float r0, r1;
         up2(r2, r0, r1);
-        acc[k] = fma2(B.y, pk2(mufu_rsqrt(r0), mufu_rsqrt(r1)), acc[k]);
+        // one chain over a stage's partners in order: two packed chains take
+        // 3 % less time, but their sums round 2 to 4e-10 of PE away from it
+        float m0, m1;
+        up2(B.y, m0, m1);
+        acc[k] = __fmaf_rn(m0, mufu_rsqrt(r0), acc[k]);
+        acc[k] = __fmaf_rn(m1, mufu_rsqrt(r1), acc[k]);
       }
     }
     const bool mine = jt < i0 + T;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      float u, v;
-      up2(acc[k], u, v);
-      const double s = (double)u + (double)v;
+      const double s = (double)acc[k];
       if (mine) own[k] += s;
       else once[k] += s;
     }
