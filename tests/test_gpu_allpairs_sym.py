@@ -28,7 +28,7 @@ def _forces(pos, eps=EPS):
 # size and ragged last tiles and chunks
 @pytest.mark.parametrize("n", [127, 128, 129, 1184, 1185, 2047, 2048, 2049, 2304, 2305, 2559, 2560, 2561,
                                4097, 8191, 8192, 8193, 8448, 8449, 16384, 16385, 24576, 24577,
-                               65536, 65537, 131073])
+                               65536, 65537, 163840, 163841])
 @pytest.mark.parametrize("masses", ["equal", "spread"])
 def test_sizes_vs_fp64(n, masses):
     pos, _ = ic.two_disks(n, seed=n)
