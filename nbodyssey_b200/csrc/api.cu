@@ -335,10 +335,13 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
     NB_TRY(launch_allpairs(w, a, st));
     return mark(pm, NB_PHASE_WALK, st);
   }
-  NB_TRY(launch_prep(w, a, true, false, st));
+  // the cluster sort finds the bounding box itself: without a kick nothing is
+  // left to prepare
+  const bool cluster = sort_in_cluster(a.n, a.key_bits);
+  if (!cluster || a.kick_drift) NB_TRY(launch_prep(w, a, !cluster, false, st));
   if (a.after_prep) NB_CUDA(cudaEventRecord(a.after_prep, st));
   NB_TRY(mark(pm, NB_PHASE_PREP, st));
-  if (sort_in_cluster(a.n, a.key_bits)) {
+  if (cluster) {
     // the keys are made in the sort's launch: their phase is the event's own
     NB_TRY(mark(pm, NB_PHASE_MORTON, st));
     NB_TRY(launch_sort_cluster(w, a, st));

@@ -437,7 +437,8 @@ int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// Morton keys and the whole sort in one launch, for n up to kClusterMax: a
+// Bounding box, Morton keys and the whole sort in one launch, for n up to
+// kClusterMax: a
 // cluster of 16 CTAs holds all keys and values in its shared memory, ranks its
 // slice of them each pass as the onesweep kernel does, sends its digit counts
 // to the others over distributed shared memory in place of the look-back, and
@@ -498,8 +499,7 @@ __host__ __device__ constexpr size_t cluster_sort_smem(int slice) {
 
 template <typename K>
 __global__ void __launch_bounds__(kClusterThreads, 1)
-    k_sort_cluster(const float4* __restrict__ pos, int n, const int* __restrict__ bbox,
-                   K* __restrict__ kout, uint32_t* __restrict__ vout,
+    k_sort_cluster(const float4* __restrict__ pos, int n, K* __restrict__ kout, uint32_t* __restrict__ vout,
                    float4* __restrict__ pos_sorted, int slice, uint32_t slice_inv, int passes,
                    unsigned* err) {
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -520,26 +520,73 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   const int items = (slice + kClusterThreads - 1) / kClusterThreads;
   const int seg = warp * items * 32 + lane;
   for (int i = tid; i < kClusterWarps * kSortRadix; i += kClusterThreads) s_match[i] = 0u;
-  cluster.barrier_arrive();   // waited for before the first remote store: every CTA has started
+  cluster.barrier_arrive();   // waited for before the first remote store
   chain_release();
   chain_wait();
 
   K key[kClusterItems];
   uint32_t val[kClusterItems];
   {
-    const float lx = ord2f(bbox[0]), ly = ord2f(bbox[1]), lz = ord2f(bbox[2]);
-    const float hx = ord2f(bbox[3]), hy = ord2f(bbox[4]), hz = ord2f(bbox[5]);
-    const float ext =
-        fmaxf(__fsub_rn(hx, lx), fmaxf(__fsub_rn(hy, ly), __fsub_rn(hz, lz)));
+    // the bounding box: this CTA's particles, then all CTAs' (min / max are
+    // order-independent)
+    float4 p[kClusterItems];
+    int r[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
+                (int)0x80000000};
+#pragma unroll
+    for (int k = 0; k < kClusterItems; ++k)
+      if (k < items && seg + 32 * k < count) p[k] = pos[first + seg + 32 * k];
+#pragma unroll
+    for (int k = 0; k < kClusterItems; ++k) {
+      if (k < items && seg + 32 * k < count) {
+        const int o[3] = {f2ord(p[k].x), f2ord(p[k].y), f2ord(p[k].z)};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          r[c] = min(r[c], o[c]);
+          r[c + 3] = max(r[c + 3], o[c]);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      r[c] = __reduce_min_sync(0xffffffffu, r[c]);
+      r[c + 3] = __reduce_max_sync(0xffffffffu, r[c + 3]);
+    }
+    int* s_red = reinterpret_cast<int*>(s_part);   // [warps][6], then every CTA's [6]
+    int* s_box = s_red + 6 * kClusterWarps;
+    if (lane == 0) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) s_red[6 * warp + c] = r[c];
+    }
+    cluster.barrier_wait();   // every CTA has started
+    __syncthreads();
+    if (tid < 6 * kClusterCtas) {   // component c to CTA `to`
+      const int c = tid % 6, to = tid / 6;
+      int v = s_red[c];
+      for (int w = 1; w < kClusterWarps; ++w)
+        v = c < 3 ? min(v, s_red[6 * w + c]) : max(v, s_red[6 * w + c]);
+      cluster.map_shared_rank(s_box, to)[6 * cta + c] = v;
+    }
+    cluster.sync();
+    float b[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      const int mine = lane < kClusterCtas ? s_box[6 * lane + c]
+                                           : (c < 3 ? 0x7fffffff : (int)0x80000000);
+      b[c] = ord2f(c < 3 ? __reduce_min_sync(0xffffffffu, mine)
+                         : __reduce_max_sync(0xffffffffu, mine));
+    }
+    const float ext = fmaxf(__fsub_rn(b[3], b[0]),
+                            fmaxf(__fsub_rn(b[4], b[1]), __fsub_rn(b[5], b[2])));
     const float inv = ext > 0.f ? __frcp_rn(ext) : 0.f;
 #pragma unroll
     for (int k = 0; k < kClusterItems; ++k) {
       const int i = seg + 32 * k;
       if (k < items && i < count) {
-        key[k] = morton_key<K>(pos[first + i], lx, ly, lz, inv);
+        key[k] = morton_key<K>(p[k], b[0], b[1], b[2], inv);
         val[k] = (uint32_t)(first + i);
       }
     }
+    __syncthreads();   // s_part is reused
   }
   for (int ps = 0; ps < passes; ++ps) {
     const int shift = 8 * ps;
@@ -604,7 +651,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       col[w * kSortRadix] = (uint16_t)before;
       before += c;
     }
-    if (ps == 0) cluster.barrier_wait();
     // this CTA's counts to every CTA (stored there: a load from another SM's
     // shared memory would wait its whole latency)
 #pragma unroll
@@ -752,7 +798,7 @@ static int cluster_sort(Workspace& w, const StepArgs& a, cudaStream_t st) {
   cfg.stream = st;
   chained_attribute(st, &cfg, at);
   NB_CUDA(cudaLaunchKernelEx(&cfg, k_sort_cluster<K>, (const float4*)a.pos, a.n,
-                             (const int*)w.bbox, (K*)w.keys, w.vals, w.pos_sorted, slice, inv,
+                             (K*)w.keys, w.vals, w.pos_sorted, slice, inv,
                              sort_passes(a.key_bits), w.err));
   return NB_OK;
 }

@@ -195,7 +195,7 @@ int launch_prep(Workspace& w, const StepArgs& s, bool bbox, bool pack,
   a.src = pack ? w.src : nullptr;
   a.zero = nullptr;
   a.zero_words = 0;
-  if (bbox && !sort_in_cluster(s.n, s.key_bits)) {
+  if (bbox) {
     a.zero = w.hist;   // hist, tile counters and status are one allocation
     // histograms, tile counters, and the tile status words of the passes
     // this key width sorts with (pass p's words follow pass p - 1's)

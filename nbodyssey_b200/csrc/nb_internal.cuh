@@ -194,7 +194,7 @@ int launch_prep(Workspace& w, const StepArgs& a, bool bbox, bool pack,
                 cudaStream_t st);
 int launch_morton(Workspace& w, const StepArgs& a, cudaStream_t st);
 int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st);
-// Morton keys and sort in one launch, for sizes that fit a cluster's shared
+// Bounding box, Morton keys and sort in one launch, for sizes that fit a cluster's shared
 // memory (on a device that can hold it); the sort scratch is not used
 bool sort_in_cluster(int n, int key_bits);
 int launch_sort_cluster(Workspace& w, const StepArgs& a, cudaStream_t st);
