@@ -317,7 +317,9 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   if (force == NB_FORCE_AUTO)
     force = resolve_force_tuned(force, a.n, std::sqrt(a.theta2), a.traverse);
   // workspace growth (allocation, host side) stays outside the timed region
-  if (force == NB_FORCE_NAIVE) NB_TRY(ws_reserve_naive(w, a.n));
+  if (force == NB_FORCE_NAIVE)
+    NB_TRY(allpairs_packed(a) ? ws_reserve_allpairs(w, a.n, allpairs_geometry(a.n))
+                              : ws_reserve_naive(w, a.n));
   else if (a.n >= 2) NB_TRY(ws_reserve(w, a.n, a.key_bits));
   if (pm) NB_CUDA(cudaEventRecord(pm->start, st));
   if (force == NB_FORCE_BH && a.n < 2) {
@@ -327,8 +329,8 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
     return mark(pm, NB_PHASE_WALK, st);
   }
   if (force == NB_FORCE_NAIVE) {
-    // up to kSymMax the kernels read the positions themselves: nothing to pack
-    const bool pack = a.n > kSymMax;
+    // most calls' kernels read the positions themselves: nothing to pack
+    const bool pack = allpairs_packed(a);
     if (pack || a.kick_drift) NB_TRY(launch_prep(w, a, false, pack, st));
     if (a.after_prep) NB_CUDA(cudaEventRecord(a.after_prep, st));
     NB_TRY(mark(pm, NB_PHASE_PREP, st));

@@ -332,7 +332,14 @@ int launch_allpairs_geom(Workspace& w, const StepArgs& s, const APGeom& g,
   return NB_OK;
 }
 
+// Above kSymMax, and for forces written over the positions themselves: the
+// tiled kernel reads its sources from the packed copy, and a tile's targets
+// before any of its forces is written; the other kernels read all positions
+// to the end.
+bool allpairs_packed(const StepArgs& s) { return s.n > kSymMax || s.acc == s.pos; }
+
 int launch_allpairs(Workspace& w, const StepArgs& s, cudaStream_t st) {
+  if (allpairs_packed(s)) return launch_allpairs_geom(w, s, allpairs_geometry(s.n), st);
   if (s.n < kSymMin) {
     APArgs a{};
     a.n = s.n;
@@ -344,10 +351,8 @@ int launch_allpairs(Workspace& w, const StepArgs& s, cudaStream_t st) {
     a.vel = s.kick_after ? s.vel : nullptr;
     return launch_allpairs_small(a, st);
   }
-  if (allpairs_sym(s.n))
-    return launch_allpairs_sym(s.n, s.pos, s.acc, s.kick_after ? s.vel : nullptr, s.eps2, s.G,
-                               s.half_dt, w.part, (size_t)w.part_cap, st);
-  return launch_allpairs_geom(w, s, allpairs_geometry(s.n), st);
+  return launch_allpairs_sym(s.n, s.pos, s.acc, s.kick_after ? s.vel : nullptr, s.eps2, s.G,
+                             s.half_dt, w.part, (size_t)w.part_cap, st);
 }
 
 // ---------------------------------------------------------------------------

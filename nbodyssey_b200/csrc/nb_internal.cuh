@@ -207,6 +207,7 @@ int launch_walk(Workspace& w, const StepArgs& a, cudaStream_t st);
 // permutation of the workspace's last tree, or the identity without one
 int launch_gather_part(Workspace& w, const StepArgs& a, const float4* sorted,
                        bool use_perm, cudaStream_t st);
+bool allpairs_packed(const StepArgs& a);   // sources from the packed copy
 int launch_allpairs(Workspace& w, const StepArgs& a, cudaStream_t st);
 // energy: {E, KE, PE, Px, Py, Pz} into w.eout (device); positions hi (+lo
 // for the kinetic part is not needed).

@@ -80,3 +80,29 @@ def test_batches_and_small_scratch_give_the_same_bits():
             srv.wait(rid, 120)
             q, w = srv.result(rid)
             assert np.array_equal(q, p) and np.array_equal(w, v)
+
+
+@pytest.mark.parametrize("n", [1000, 2559, 2560, 9000])
+def test_forces_over_the_positions(n):
+    """nb_compute_forces_dev with one buffer for positions and forces: each
+    target's force comes from the positions, none from forces already written."""
+    import ctypes
+
+    import torch
+
+    from nbodyssey_b200 import _lib as L
+    lib = L.load()
+    pos, _ = ic.two_disks(n, seed=n)
+    buf = torch.from_numpy(pos).cuda()
+    prm = api.SimParams(epsilon=EPS, force="naive").to_c()
+    ws = ctypes.c_void_p()
+    L.check(lib.nb_workspace_create(ctypes.byref(ws)))
+    try:
+        ptr = ctypes.c_void_p(buf.data_ptr())
+        L.check(lib.nb_compute_forces_dev(ws, n, ptr, ptr, ctypes.byref(prm),
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        acc = buf.cpu().numpy()
+    finally:
+        L.check(lib.nb_workspace_destroy(ws))
+    r = _rel(acc[:, :3].astype(np.float64), O.allpairs_f64(pos, EPS))
+    assert np.median(r) < 2e-6 and np.percentile(r, 99) < 2e-5
