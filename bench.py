@@ -57,10 +57,11 @@ L2_FLUSH_BYTES = 256 << 20
 
 
 def bh_kernels_per_step(n, key_bits=30):
-    """Kernels of one Barnes-Hut step: prep, Morton keys, the sort passes,
-    the first build level (1024-leaf groups), one launch per later build
-    level (15 segments per CTA with 30-bit keys, 10 with 63-bit; the
-    geometry of nbodyssey_b200/csrc/k_lbvh.cu) and the walk."""
+    """Kernels of one Barnes-Hut step that sorts by onesweep passes: prep,
+    Morton keys, the sort passes, the first build level, one launch per later
+    build level (as many as 1024-leaf groups need; 15 segments per CTA with
+    30-bit keys, 10 with 63-bit; the geometry of
+    nbodyssey_b200/csrc/k_lbvh.cu) and the walk."""
     passes = 4 if key_bits == 30 else 8
     fan = 15 if key_bits == 30 else 10
     groups = (n + 1023) // 1024
@@ -69,6 +70,23 @@ def bh_kernels_per_step(n, key_bits=30):
         groups = (groups + fan - 1) // fan
         levels += 1
     return 1 + 1 + passes + 1 + levels + 1
+
+
+def step_launches(n, force, key_bits=30):
+    """Kernels of one step: the Barnes-Hut chain, its keys and sort in one
+    cluster launch up to 65,536 particles (36,864 with 63-bit keys), or the
+    kick and the all-pairs launch (two from 2,560 to 2^20 particles: pairs
+    and sums; more only where the table of sums takes several passes)."""
+    if force != "bh":
+        return 3 if 2560 <= n <= 1 << 20 else 2
+    chain = bh_kernels_per_step(n, key_bits)
+    if n <= (65536 if key_bits == 30 else 36864):
+        chain -= 4 if key_bits == 30 else 8   # keys and passes in one
+    return chain
+
+
+def allpairs_kernel(n):
+    return "k_ap_small" if n < 2560 else "k_ap_sym" if n <= 1 << 20 else "k_allpairs"
 
 
 def parse_args():
@@ -454,7 +472,7 @@ def run_b200(args, rank, world, local, pg):
     if not hbm:   # the copy bandwidth measured earlier on this pool's B200s
         hbm, hbm_src = HBM_FALLBACK_GBS, "6,650 GB/s copy bandwidth (of fallback)"
     kernel = ({"pair": "k_walk_pair", "list": "k_walk_list"}.get(
-        args.walk, "k_walk_%s" % args.traverse) if args.force == "bh" else "k_allpairs")
+        args.walk, "k_walk_%s" % args.traverse) if args.force == "bh" else allpairs_kernel(args.n))
     traffic = (profiled_traffic(kernel, args.traverse, args.theta)
                if args.n == N_DEFAULT and args.force == "bh" else None)
     line = {
@@ -473,8 +491,7 @@ def run_b200(args, rank, world, local, pg):
         "phases_path": "kernel-by-kernel launches with an event between phases",
         "interactions_per_particle": inter / n,
         # the step's kernels plus the L2-flush kernel before each step
-        "gpu_launches": ((bh_kernels_per_step(n) if args.force == "bh" else 2) + 1)
-                        * args.steps,
+        "gpu_launches": (step_launches(n, args.force) + 1) * args.steps,
         "e2e": {"value": world * args.e2e_steps / e2e_s, "unit": "steps/s",
                 "h2d_bytes_per_step": 32 * n, "d2h_bytes_per_step": 32 * n,
                 "path": "nb_step_host_state: pinned host pos / vel in, a device check "
@@ -486,7 +503,8 @@ def run_b200(args, rank, world, local, pg):
                      "frac": achieved / fp32_peak, "traffic": traffic,
                      "work": ("20 flop x per-thread-criterion interactions "
                               "(%.4g per step)" % inter if args.force == "bh" else
-                              "20 flop x N^2 pairs (%.4g per step)" % inter),
+                              "20 flop x N^2 interactions (%.4g per step; up to 2^20 particles "
+                              "an unordered pair is evaluated once)" % inter),
                      "peak_source": "measured on this GPU: FP32 FMA calibration "
                                     "kernel (scalar %.1f, packed f32x2 %.1f TFLOP/s)" %
                                     (ps.value, pp.value)},
@@ -614,7 +632,7 @@ def run_shard(args, rank, world, local, pg):
         "interactions_per_particle": inter / n,
         # per step: the step's kernels on each rank plus the gather kernel
         # (the flush and the all-gather are torch / NCCL kernels)
-        "gpu_launches": world * (bh_kernels_per_step(n) + 1) * args.steps,
+        "gpu_launches": world * (step_launches(n, "bh") + 1) * args.steps,
         "e2e": {"value": args.e2e_steps / e2e_s, "unit": "steps/s",
                 "h2d_bytes_per_step": 48 * n * world, "d2h_bytes_per_step": 48 * n * world,
                 "path": "each rank: pinned host state in, ShardedSimulation.step, "
