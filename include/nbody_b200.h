@@ -108,6 +108,8 @@ NB_API int nb_measure_fp32_peak(double* tflops_scalar, double* tflops_packed);
  * it.  NBODY_B200_TUNE=off keeps the defaults.  The device-pointer entry
  * points use the current table and never measure.  The shape decides only
  * the launch: the same table gives the same bits however it was obtained.
+ * All-pairs calls of up to 2^20 particles take kernels that the table does not
+ * govern; their sums follow from n alone.
  * ==================================================================== */
 #define NB_TUNE_VERSION 2
 #define NB_TUNE_BUCKETS 16 /* size bucket b: n < 2^(10+b) (the last: any n) */

@@ -38,8 +38,8 @@
 // excludes a lane contribute with mass 0.  A stack that would overflow hands
 // the warp to a depth-first walk of the same semantics over the same records.
 //
-// Bound: with many warps, issue slots (76 % busy) and the shared-memory pipe
-// (77 %) together, the FMA pipe 52 %: 0.94 ms and 773M warp instructions at 1M
+// Bound: with many warps, issue slots (70 % busy) and the shared-memory pipe
+// (72 %) together, the FMA pipe 51 %: 0.94 ms and 725M warp instructions at 1M
 // particles, theta 0.5, warp semantics (0.998 ms and 811M with dominant-axis
 // extremes, a 64-bit vote mask and pair-interleaved entries).  With few, the
 // latency of a step, the record loads above all: the next step's are issued
