@@ -42,15 +42,18 @@ int launch_ens_step(EnsArgs& e, const BuildPlan& plan, const EnsAllPairs& ap, bo
     NB_CUDA(cudaStreamWaitEvent(fork.aux, fork.start, 0));
     NB_TRY(launch_ens_allpairs(e, ap, fork.aux));
   }
-  NB_TRY(launch_ens_morton(e, st));
-  NB_TRY(launch_ens_sort(e, st));
-  NB_TRY(launch_ens_levels(e, plan, st));
-  NB_TRY(launch_walk_pair_ens(e, fork, st));
+  auto tree = [&]() {
+    NB_TRY(launch_ens_morton(e, st));
+    NB_TRY(launch_ens_sort(e, st));
+    NB_TRY(launch_ens_levels(e, plan, st));
+    return launch_walk_pair_ens(e, fork, st);
+  };
+  const int rc = tree();   // joined below whether or not it could be launched
   if (beside || (e.walk_nitems[0] > 0 && e.walk_nitems[1] > 0)) {
     NB_CUDA(cudaEventRecord(fork.done, fork.aux));
     NB_CUDA(cudaStreamWaitEvent(st, fork.done, 0));
   }
-  return NB_OK;
+  return rc;
 }
 
 }  // namespace nb

@@ -630,7 +630,7 @@ void plan_walk_queue(const SimDesc* sims, int nsims, std::vector<int> items[2]) 
 // are both; the caller joins it.
 int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st) {
   NB_CUDA(cudaMemsetAsync(e.walk_ctr, 0, 2 * sizeof(int), st));
-  const int cap = device_sm_count() * 8;   // 8 resident blocks of 4 warps per SM
+  const int cap = device_sm_count() * 8;   // blocks of 4 warps; 6 per SM run at once
   const bool both = e.walk_nitems[0] > 0 && e.walk_nitems[1] > 0;
   if (both) {
     NB_CUDA(cudaEventRecord(fork.walks, st));
