@@ -77,7 +77,6 @@ struct nb_ensemble {
   std::vector<int> walk_items[2];   // the walk queue (host copy)
   Workspace ews;               // energy scratch
   double* d_energy = nullptr;  // [nsims][6]
-  unsigned* h_err = nullptr;   // pinned
   bool primed = false;
   bool any_tree = false;       // some simulation uses the tree pipeline
   bool use_graphs = true;
@@ -110,7 +109,6 @@ void ens_free(nb_ensemble* h) {
     if (ev) cudaEventDestroy(ev);
   for (void* p : h->allocs) cudaFree(p);
   ws_free(h->ews);
-  if (h->h_err) cudaFreeHost(h->h_err);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -164,12 +162,12 @@ int ens_capture(nb_ensemble* h) {
 }
 
 // Waits for the stream (its error word is the last thing on it) and reports
-// what the kernels raised.
+// what the kernels raised.  The word lands on the stack: a pinned one would
+// take 1 to 3 ms of the ensemble's creation.
 int ens_device_error(nb_ensemble* h) {
-  NB_CUDA(cudaMemcpyAsync(h->h_err, h->e.err, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                          h->stream));
+  unsigned v = 0;
+  NB_CUDA(cudaMemcpyAsync(&v, h->e.err, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
   NB_CUDA(cudaStreamSynchronize(h->stream));
-  const unsigned v = *h->h_err;
   if (v) {
     NB_CUDA(cudaMemsetAsync(h->e.err, 0, sizeof(unsigned), h->stream));
     NB_CUDA(cudaStreamSynchronize(h->stream));
@@ -300,7 +298,6 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     }
     if ((rc = ens_alloc(h, &h->d_energy, 6 * (size_t)nsims)) != NB_OK) break;
     cudaError_t ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaMallocHost((void**)&h->h_err, sizeof(unsigned));
     if (ce != cudaSuccess) { rc = set_error(NB_ERR_CUDA, cudaGetErrorString(ce)); break; }
     if ((rc = h->fork.create()) != NB_OK) break;
     cudaStream_t st = h->stream;
