@@ -57,7 +57,7 @@ constexpr int kSymThreads = 32 * kSymWarps;
 SymGeom allpairs_sym_geometry(int n) {
   SymGeom g;
   g.tile = n <= 16384 ? 256 : n <= 24576 ? 512 : n <= 65536 ? 1024 : n <= 163840 ? 2048 : 4096;
-  g.chunk = std::max(256, g.tile / 2);
+  g.chunk = std::max(256, g.tile / 2);   // at most kSymChunkMax
   g.tiles = (n + g.tile - 1) / g.tile;
   g.chunks = (n + g.chunk - 1) / g.chunk;
   return g;
@@ -321,9 +321,14 @@ __global__ void __launch_bounds__(kSymThreads) k_ap_sym_reduce_batch(
   sym_reduce(a, it.y, kick != 0);
 }
 
-static int sym_smem(int chunk) {
+// Dynamic shared memory of an item: below the 48 KB that every launch may ask
+// for, so no launch raises the kernels' limit -- it belongs to the function, and
+// a smaller call of another thread would lower it between a raise and its launch.
+constexpr int kSymChunkMax = 2048;
+static constexpr int sym_smem(int chunk) {
   return (kSymWarps * 3 * kSymSub + 3 * chunk) * (int)sizeof(float);
 }
+static_assert(sym_smem(kSymChunkMax) <= 48 * 1024, "no opt-in shared memory");
 
 // Fields that depend on n alone.
 static SymArgs sym_args(int n) {
@@ -350,7 +355,6 @@ int launch_allpairs_sym(int n, const float4* pos, float4* acc, float4* vel, floa
   a.G = G;
   a.half_dt = half_dt;
   const int smem = sym_smem(a.chunk);
-  NB_CUDA(cudaFuncSetAttribute(k_ap_sym, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int per = a.tile / a.chunk;
   for (a.ta = 0; a.ta < a.tiles; a.ta = a.tb) {
     a.tb = std::min(a.tiles, a.ta + rows);
@@ -460,11 +464,8 @@ int SymPlan::launch(const EnsArgs& e, cudaStream_t st) const {
   const int2* d_blocks = reinterpret_cast<const int2*>(d_args + args.size());
   const int nargs = (int)args.size();
   for (const Pass& p : passes) {
-    const int smem = sym_smem(p.chunk);
-    NB_CUDA(cudaFuncSetAttribute(k_ap_sym_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem));
-    k_ap_sym_batch<<<p.items, kSymThreads, smem, st>>>(d_args, nargs, d_items + p.first_item,
-                                                       e.err);
+    k_ap_sym_batch<<<p.items, kSymThreads, sym_smem(p.chunk), st>>>(
+        d_args, nargs, d_items + p.first_item, e.err);
     NB_CUDA(cudaGetLastError());
     k_ap_sym_reduce_batch<<<p.blocks, kSymThreads, 0, st>>>(
         d_args, nargs, d_blocks + p.first_block, e.kick_after ? 1 : 0, e.err);
