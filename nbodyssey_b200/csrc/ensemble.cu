@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "fork_join.h"
 #include "nb_internal.cuh"
 
 namespace nb {
@@ -36,24 +37,25 @@ int launch_ens_step(EnsArgs& e, const BuildPlan& plan, const EnsAllPairs& ap, bo
                     const EnsFork& fork, cudaStream_t st) {
   NB_TRY(launch_ens_prep(e, st));
   if (!any_tree) return launch_ens_allpairs(e, ap, st);
-  const bool beside = !ap.args.empty() || !ap.sym.args.empty();
-  if (beside) {
-    NB_CUDA(cudaEventRecord(fork.start, st));
-    NB_CUDA(cudaStreamWaitEvent(fork.aux, fork.start, 0));
-    NB_TRY(launch_ens_allpairs(e, ap, fork.aux));
-  }
-  auto tree = [&]() {
-    NB_TRY(launch_ens_morton(e, st));
-    NB_TRY(launch_ens_sort(e, st));
-    NB_TRY(launch_ens_levels(e, plan, st));
-    return launch_walk_pair_ens(e, fork, st);
-  };
-  const int rc = tree();   // joined below whether or not it could be launched
-  if (beside || (e.walk_nitems[0] > 0 && e.walk_nitems[1] > 0)) {
-    NB_CUDA(cudaEventRecord(fork.done, fork.aux));
-    NB_CUDA(cudaStreamWaitEvent(st, fork.done, 0));
-  }
-  return rc;
+  return run_forked(
+      !ap.args.empty() || !ap.sym.args.empty(),
+      [&]() {
+        NB_CUDA(cudaEventRecord(fork.start, st));
+        NB_CUDA(cudaStreamWaitEvent(fork.aux, fork.start, 0));
+        return NB_OK;
+      },
+      [&]() { return launch_ens_allpairs(e, ap, fork.aux); },
+      [&](bool* used) {
+        NB_TRY(launch_ens_morton(e, st));
+        NB_TRY(launch_ens_sort(e, st));
+        NB_TRY(launch_ens_levels(e, plan, st));
+        return launch_walk_pair_ens(e, fork, st, used);
+      },
+      [&]() {
+        NB_CUDA(cudaEventRecord(fork.done, fork.aux));
+        NB_CUDA(cudaStreamWaitEvent(st, fork.done, 0));
+        return NB_OK;
+      });
 }
 
 }  // namespace nb

@@ -627,14 +627,15 @@ void plan_walk_queue(const SimDesc* sims, int nsims, std::vector<int> items[2]) 
 }
 
 // Thread semantics' walk, the longer one, goes to the fork's stream when there
-// are both; the caller joins it.
-int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st) {
+// are both; `forked` is then set and the caller joins it.
+int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st, bool* forked) {
   NB_CUDA(cudaMemsetAsync(e.walk_ctr, 0, 2 * sizeof(int), st));
   const int cap = device_sm_count() * 8;   // blocks of 4 warps; 6 per SM run at once
   const bool both = e.walk_nitems[0] > 0 && e.walk_nitems[1] > 0;
   if (both) {
     NB_CUDA(cudaEventRecord(fork.walks, st));
     NB_CUDA(cudaStreamWaitEvent(fork.aux, fork.walks, 0));
+    *forked = true;
   }
   for (int q = 1; q >= 0; --q) {
     const int n = e.walk_nitems[q];

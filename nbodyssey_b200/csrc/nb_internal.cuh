@@ -586,7 +586,7 @@ struct EnsFork {
 // the device.
 int launch_ens_step(EnsArgs& e, const BuildPlan& plan, const EnsAllPairs& ap, bool any_tree,
                     const EnsFork& fork, cudaStream_t st);
-int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st);
+int launch_walk_pair_ens(const EnsArgs& e, const EnsFork& fork, cudaStream_t st, bool* forked);
 // Host: the walk queue of a simulation table (the Barnes-Hut simulations'
 // 32-slot blocks per semantics, costliest simulation first: larger n and
 // smaller theta walk longer); items[0] / items[1] get the warp / thread
