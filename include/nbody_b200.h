@@ -103,7 +103,7 @@ NB_API int nb_measure_fp32_peak(double* tflops_scalar, double* tflops_packed);
  * all-pairs / Barnes-Hut crossover NB_FORCE_AUTO uses, measured on the device
  * at first use: the first nb_sim_create / nb_ensemble_create /
  * nb_server_create on a device loads the cache file
- * ($NBODY_B200_TUNE_CACHE, else ~/.cache/nbodyssey_b200/tune_<device>_<SMs>sm_v2.bin)
+ * ($NBODY_B200_TUNE_CACHE, else ~/.cache/nbodyssey_b200/tune_<device>_<SMs>sm_v3.bin)
  * or, when there is none, measures the table (about a second) and writes
  * it.  NBODY_B200_TUNE=off keeps the defaults.  The device-pointer entry
  * points use the current table and never measure.  The shape decides only
@@ -111,7 +111,7 @@ NB_API int nb_measure_fp32_peak(double* tflops_scalar, double* tflops_packed);
  * All-pairs calls of up to 2^20 particles take kernels that the table does not
  * govern; their sums follow from n alone.
  * ==================================================================== */
-#define NB_TUNE_VERSION 2
+#define NB_TUNE_VERSION 3
 #define NB_TUNE_BUCKETS 16 /* size bucket b: n < 2^(10+b) (the last: any n) */
 #define NB_TUNE_THETAS 3   /* crossover per theta class 0.3, 0.5, 0.7 */
 typedef struct nb_tune_table {

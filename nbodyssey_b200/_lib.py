@@ -54,7 +54,7 @@ class nb_params(ctypes.Structure):
                 ("walk_kernel", ctypes.c_int32)]
 
 
-NB_TUNE_VERSION = 2
+NB_TUNE_VERSION = 3
 NB_TUNE_BUCKETS = 16
 NB_TUNE_THETAS = 3
 
