@@ -391,9 +391,7 @@ size_t ap_region_f4(int n) {
   const size_t npad = (size_t)(n + kSrcTile - 1) / kSrcTile * kSrcTile;
   const size_t part = g.jsplit > 1 ? (size_t)g.jsplit * n : 0;
   const size_t tick = ((size_t)g.itiles + 3) / 4;
-  size_t f4 = npad + part + tick;
-  if (allpairs_sym(n)) f4 = std::max(f4, allpairs_sym_row_f4(n));
-  return (f4 + 15) / 16 * 16;
+  return (npad + part + tick + 15) / 16 * 16;
 }
 
 size_t ap_region_whole_f4(int n) {
@@ -438,7 +436,10 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
     a.half_dt = d.half_dt;
     const size_t r = region_of ? region_of[s] : next;
     const size_t size = region_cap ? region_cap[s] : size_of(d.n);
-    if (ap_region_f4(d.n) > size) {   // the table changed
+    const size_t least = allpairs_sym(d.n) ? allpairs_sym_least_f4(d.n)
+                         : d.n < kSymMin   ? 0
+                                           : ap_region_f4(d.n);
+    if (least > size) {   // the table changed
       if (too_small) ++*too_small;
       continue;
     }

@@ -31,8 +31,8 @@
 // a fixed order -- tiles before its own, then the chunks from its own tile on
 // -- and applies the closing kick, so results repeat bit for bit.  A table that
 // would be larger than the scratch at hand is used for a few rows of tiles at
-// a time, the running sums kept in `acc`; the order, and so every bit, is the
-// same.
+// a time, or for a few chunks of one row, the running sums kept in `acc`; the
+// order, and so every bit, is the same.
 #include <algorithm>
 #include <vector>
 
@@ -70,6 +70,11 @@ bool allpairs_sym(int n) { return n >= kSymMin && n <= kSymMax; }
 size_t allpairs_sym_row_f4(int n) {
   const SymGeom g = allpairs_sym_geometry(n);
   return (size_t)n + (size_t)g.chunks * g.tile;
+}
+
+size_t allpairs_sym_least_f4(int n) {
+  const SymGeom g = allpairs_sym_geometry(n);
+  return (size_t)g.chunk + g.tile;
 }
 
 // A lane's targets (negated positions and masses, each in both halves of a
@@ -230,13 +235,13 @@ __device__ __forceinline__ void sym_item(const SymArgs& a, int I, int c) {
 // chunk counts add up to the same number, so the grid is a rectangle.
 __global__ void __launch_bounds__(kSymThreads, 2) k_ap_sym(SymArgs a) {
   const int per = a.tile / a.chunk;
-  int I = a.ta + blockIdx.y, x = blockIdx.x;
+  int I = a.ta + blockIdx.y, x = blockIdx.x + max(0, a.ca - I * per);
   const int last = a.tb - 1 - blockIdx.y;
-  if (x >= a.chunks - I * per) {
-    x -= a.chunks - I * per;
+  if (x >= a.cb - I * per) {
+    x -= a.cb - I * per;
     if (last <= I) return;   // the middle row of an odd count
     I = last;
-    if (x >= a.chunks - I * per) return;
+    if (x >= a.cb - I * per) return;
   }
   sym_item(a, I, I * per + x);
 }
@@ -250,7 +255,8 @@ __global__ void __launch_bounds__(kSymThreads, 2) k_ap_sym_batch(
   SymArgs a{};
   if (ok) {
     a = args[it.x];
-    ok = it.y >= a.ta && it.y < a.tb && it.z >= it.y * (a.tile / a.chunk) && it.z < a.chunks;
+    ok = it.y >= a.ta && it.y < a.tb && it.z >= max(it.y * (a.tile / a.chunk), a.ca) &&
+         it.z < a.cb;
   }
   if (!ok) {   // a stale or corrupt item: skipped, reported
     if (threadIdx.x == 0) raise_err(err, NB_DEVERR_QUEUE);
@@ -259,14 +265,14 @@ __global__ void __launch_bounds__(kSymThreads, 2) k_ap_sym_batch(
   sym_item(a, it.y, it.z);
 }
 
-// Adds target t's partials of tiles [ta, tb); the launch that holds its own
-// tile ends its sum.
+// Adds target t's partials of tiles [ta, tb) and chunks [ca, cb); the pass that
+// holds its own tile's last chunk ends its sum.
 __device__ __forceinline__ void sym_reduce(const SymArgs& a, int block, bool kick) {
   const int t = a.ta * a.tile + block * kSymThreads + threadIdx.x;
   if (t >= a.n) return;
   const int T = t / a.tile;
   float3 s = make_float3(0.f, 0.f, 0.f);
-  if (a.ta > 0) {
+  if (a.ta > 0 || a.ca > 0) {
     const float4 r = a.acc[t];
     s = make_float3(r.x, r.y, r.z);
   }
@@ -286,14 +292,20 @@ __device__ __forceinline__ void sym_reduce(const SymArgs& a, int block, bool kic
       }
     }
   };
-  add(a.row + t, a.n, min(T, a.tb) - a.ta);
+  // the pass holds this target's rows when it holds its chunk
+  const bool rows = t >= a.ca * a.chunk && t < a.cb * a.chunk;
+  add(a.row + t, a.n, rows ? min(T, a.tb) - a.ta : 0);
   if (T >= a.tb) {
     a.acc[t] = make_float4(s.x, s.y, s.z, 0.f);
     return;
   }
   const size_t width = (size_t)(a.tb - a.ta) * a.tile;
-  const int c0 = T * (a.tile / a.chunk);
-  add(a.col + c0 * width + (t - a.ta * a.tile), width, a.chunks - c0);
+  const int c0 = max(T * (a.tile / a.chunk), a.ca);
+  add(a.col + c0 * width + (t - a.ta * a.tile), width, a.cb - c0);
+  if (a.cb < a.chunks) {
+    a.acc[t] = make_float4(s.x, s.y, s.z, 0.f);
+    return;
+  }
   const float4 acc = make_float4(a.G * s.x, a.G * s.y, a.G * s.z, 0.f);
   a.acc[t] = acc;
   if (kick && a.vel) {
@@ -342,40 +354,74 @@ static SymArgs sym_args(int n) {
   return a;
 }
 
+// Calls fn for each pass over a table of scratch_f4 float4: as many rows of
+// tiles as it holds, all their chunks, or, when it does not hold one row, as
+// many chunks of one.
+template <typename F>
+static int sym_passes(SymArgs a, size_t scratch_f4, F fn) {
+  const size_t rows = scratch_f4 / allpairs_sym_row_f4(a.n);
+  if (rows > 0) {
+    a.ca = 0;
+    a.cb = a.chunks;
+    for (a.ta = 0; a.ta < a.tiles; a.ta = a.tb) {
+      a.tb = (int)std::min<size_t>(a.tiles, a.ta + rows);
+      NB_TRY(fn(a));
+    }
+    return NB_OK;
+  }
+  const int span = (int)(scratch_f4 / allpairs_sym_least_f4(a.n));
+  if (span < 1) return set_error(NB_ERR_NOMEM, "all-pairs scratch too small");
+  for (a.ta = 0; a.ta < a.tiles; ++a.ta) {
+    a.tb = a.ta + 1;
+    for (a.ca = a.ta * (a.tile / a.chunk); a.ca < a.chunks; a.ca = a.cb) {
+      a.cb = std::min(a.chunks, a.ca + span);
+      NB_TRY(fn(a));
+    }
+  }
+  return NB_OK;
+}
+
+// The pass's table in `scratch`: row [tb - ta][n], col [chunks][(tb - ta) tile].
+// A pass over some chunks of one row holds their part of both; the kernels index
+// from where chunk 0 would lie.
+static void sym_place(SymArgs& a, float4* scratch) {
+  const size_t cnt = a.tb - a.ta;
+  const bool all = a.ca == 0 && a.cb == a.chunks;
+  const size_t row_f4 = all ? cnt * a.n : (size_t)(a.cb - a.ca) * a.chunk;
+  a.row = scratch - (size_t)a.ca * a.chunk;
+  a.col = scratch + row_f4 - (size_t)a.ca * cnt * a.tile;
+}
+
 int launch_allpairs_sym(int n, const float4* pos, float4* acc, float4* vel, float eps2,
                         float G, float half_dt, float4* scratch, size_t scratch_f4,
                         cudaStream_t st) {
-  SymArgs a = sym_args(n);
-  const int rows = (int)std::min<size_t>(a.tiles, scratch_f4 / allpairs_sym_row_f4(n));
-  if (rows < 1) return set_error(NB_ERR_NOMEM, "all-pairs scratch too small");
-  a.pos = pos;
-  a.acc = acc;
-  a.vel = vel;
-  a.eps2 = eps2;
-  a.G = G;
-  a.half_dt = half_dt;
-  const int smem = sym_smem(a.chunk);
-  const int per = a.tile / a.chunk;
-  for (a.ta = 0; a.ta < a.tiles; a.ta = a.tb) {
-    a.tb = std::min(a.tiles, a.ta + rows);
+  SymArgs base = sym_args(n);
+  base.pos = pos;
+  base.acc = acc;
+  base.vel = vel;
+  base.eps2 = eps2;
+  base.G = G;
+  base.half_dt = half_dt;
+  const int smem = sym_smem(base.chunk);
+  const int per = base.tile / base.chunk;
+  return sym_passes(base, scratch_f4, [&](SymArgs a) {
+    sym_place(a, scratch);
     const int cnt = a.tb - a.ta;
-    a.row = scratch;
-    a.col = scratch + (size_t)cnt * n;
     // chunks of the first and the last row of a folded pair together
-    int wide = a.chunks - a.ta * per;
+    int wide = a.cb - std::max(a.ca, a.ta * per);
     if (cnt > 1) wide += a.chunks - (a.tb - 1) * per;
     k_ap_sym<<<dim3(wide, (cnt + 1) / 2), kSymThreads, smem, st>>>(a);
     NB_CUDA(cudaGetLastError());
     const int left = n - a.ta * a.tile;
     k_ap_sym_reduce<<<(left + kSymThreads - 1) / kSymThreads, kSymThreads, 0, st>>>(a);
     NB_CUDA(cudaGetLastError());
-  }
-  return NB_OK;
+    return NB_OK;
+  });
 }
 
-// A simulation of a batch whose scratch is `region_f4` float4 at `region` of
-// the pool takes as many rows of tiles at a time as fit there; the batch's
-// launches of pass k hold pass k of every simulation.
+// A simulation of a batch takes its passes over the `region_f4` float4 that it
+// has at `region` of the pool; the batch's launches of pass k hold pass k of
+// every simulation.
 void SymPlan::clear() {
   args.clear();
   sim.clear();
@@ -387,19 +433,18 @@ void SymPlan::clear() {
 }
 
 void SymPlan::add(int s, const SimDesc& d, size_t at, size_t region_f4) {
-  SymArgs a = sym_args(d.n);
-  a.eps2 = d.eps2;
-  a.G = d.G;
-  a.half_dt = d.half_dt;
-  const int rows = (int)std::max<size_t>(1, std::min<size_t>(a.tiles, region_f4 / allpairs_sym_row_f4(d.n)));
+  SymArgs base = sym_args(d.n);
+  base.eps2 = d.eps2;
+  base.G = d.G;
+  base.half_dt = d.half_dt;
   int k = 0;
-  for (a.ta = 0; a.ta < a.tiles; a.ta = a.tb, ++k) {
-    a.tb = std::min(a.tiles, a.ta + rows);
+  sym_passes(base, region_f4, [&](const SymArgs& a) {   // the caller has checked the least
     args.push_back(a);
     sim.push_back(s);
     region.push_back(at);
-    pass.push_back(k);
-  }
+    pass.push_back(k++);
+    return NB_OK;
+  });
 }
 
 // Items and reduction blocks, pass by pass; larger chunks first.
@@ -416,7 +461,8 @@ void SymPlan::finish() {
       const SymArgs& a = args[i];
       const int per = a.tile / a.chunk;
       for (int I = a.ta; I < a.tb; ++I)
-        for (int c = I * per; c < a.chunks; ++c) items.push_back(make_int4(i, I, c, 0));
+        for (int c = std::max(I * per, a.ca); c < a.cb; ++c)
+          items.push_back(make_int4(i, I, c, 0));
       const int left = a.n - a.ta * a.tile;
       for (int b = 0; b < (left + kSymThreads - 1) / kSymThreads; ++b)
         blocks.push_back(make_int2(i, b));
@@ -440,8 +486,7 @@ int SymPlan::bind(const SimDesc* sims, const EnsArgs& e, float4* pool, cudaStrea
     a.pos = e.pos + d.base;
     a.acc = e.acc + d.base;
     a.vel = d.active == 1 ? e.vel + d.base : nullptr;
-    a.row = pool + region[i];
-    a.col = a.row + (size_t)(a.tb - a.ta) * a.n;
+    sym_place(a, pool + region[i]);
   }
   if (args.empty()) return NB_OK;
   // items first: 16-byte entries at the start of the allocation

@@ -364,9 +364,10 @@ struct SymGeom {
   int tiles, chunks;
 };
 SymGeom allpairs_sym_geometry(int n);
-// scratch float4 of one row of tiles; any number of rows from 1 to `tiles`
-// gives the same bits
+// scratch float4 of one row of tiles, and the least a pass runs with; any
+// amount from that on gives the same bits
 size_t allpairs_sym_row_f4(int n);
+size_t allpairs_sym_least_f4(int n);
 int launch_allpairs_sym(int n, const float4* pos, float4* acc, float4* vel, float eps2,
                         float G, float half_dt, float4* scratch, size_t scratch_f4,
                         cudaStream_t st);
@@ -476,7 +477,8 @@ struct EnsArgs {
   int* walk_ctr;
 };
 
-// Arguments of the pairs-once kernel for the tiles [ta, tb) of one simulation.
+// Arguments of the pairs-once kernel for the tiles [ta, tb) and chunks [ca, cb)
+// of one simulation.
 struct SymArgs {
   const float4* __restrict__ pos;
   float4* acc;
@@ -487,6 +489,7 @@ struct SymArgs {
   int n;
   int tile, chunk, tiles, chunks;
   int ta, tb;
+  int ca, cb;           // chunks of this pass (all, or some of one row's)
 };
 static_assert(sizeof(SymArgs) % 8 == 0, "tables of SymArgs are followed by 8-byte entries");
 
@@ -540,7 +543,8 @@ struct EnsAllPairs {
 // Pool float4 of one simulation's region (sources, partials, tickets); its
 // sources come first and must start zeroed, its tickets too.  A simulation of
 // the pairs-once kernel keeps its table of partials there, whole with
-// ap_region_whole_f4, in passes over as many rows as fit with less.
+// ap_region_whole_f4, in passes over as much of it as fits with less (the
+// tiled kernel's region always holds the least).
 size_t ap_region_f4(int n);
 size_t ap_region_whole_f4(int n);
 // Host plan of the simulations whose SimDesc.force is NB_FORCE_NAIVE and that
