@@ -164,20 +164,29 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
 }
 
 // Scratch of the pairs-once kernel: all rows of tiles up to 1 GiB, fewer when
-// that cannot be had (one row at least).
-static int ws_reserve_allpairs_sym(Workspace& w, int n) {
+// that cannot be had (one row at least).  The whole table does not grow with n
+// throughout (a larger tile makes it smaller), and a capture cannot allocate:
+// there a size that a larger call has reserved for takes the table at hand, in
+// passes over what it holds.
+static int ws_reserve_allpairs_sym(Workspace& w, int n, cudaStream_t st) {
   NB_TRY(ws_basic(w));
   const size_t row = allpairs_sym_row_f4(n);
   const size_t tiles = allpairs_sym_geometry(n).tiles;
   size_t rows = std::max<size_t>(1, std::min(tiles, ((size_t)1 << 26) / row));
-  if ((size_t)w.part_cap >= rows * row) return NB_OK;
-  for (;; rows = (rows + 1) / 2) {
-    w.part_cap = 0;
-    const int rc = dalloc(&w.part, rows * row);
-    if (rc == NB_OK) break;
-    if (rows == 1) return rc;
+  if ((size_t)w.part_cap < rows * row) {
+    if (n <= w.ap_n && is_capturing(st)) return NB_OK;
+    for (;; rows = (rows + 1) / 2) {
+      w.part_cap = 0;
+      const int rc = dalloc(&w.part, rows * row);
+      if (rc == NB_OK) break;
+      if (rows == 1) {
+        w.ap_n = 0;
+        return rc;
+      }
+    }
+    w.part_cap = (int)(rows * row);
   }
-  w.part_cap = (int)(rows * row);
+  w.ap_n = std::max(w.ap_n, n);
   return NB_OK;
 }
 
@@ -189,6 +198,7 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
     w.src_cap = npad;
   }
   size_t need = g.jsplit > 1 ? (size_t)g.jsplit * n : 1;
+  if (allpairs_sym(n)) need = std::max(need, allpairs_sym_least_f4(n));
   if (need > (size_t)w.part_cap) {
     NB_TRY(dalloc(&w.part, need));
     w.part_cap = (int)need;
@@ -199,12 +209,13 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
     NB_CUDA(cudaMemset(w.tickets, 0, itiles * sizeof(unsigned)));
     w.tickets_cap = itiles;
   }
+  if ((size_t)w.part_cap >= allpairs_sym_least_f4(n)) w.ap_n = std::max(w.ap_n, n);
   return NB_OK;
 }
 
-int ws_reserve_naive(Workspace& w, int n) {
+int ws_reserve_naive(Workspace& w, int n, cudaStream_t st) {
   if (n < kSymMin) return ws_basic(w);   // no scratch
-  if (allpairs_sym(n)) return ws_reserve_allpairs_sym(w, n);
+  if (allpairs_sym(n)) return ws_reserve_allpairs_sym(w, n, st);
   return ws_reserve_allpairs(w, n, allpairs_geometry(n));
 }
 
@@ -319,7 +330,7 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   // workspace growth (allocation, host side) stays outside the timed region
   if (force == NB_FORCE_NAIVE)
     NB_TRY(allpairs_packed(a) ? ws_reserve_allpairs(w, a.n, allpairs_geometry(a.n))
-                              : ws_reserve_naive(w, a.n));
+                              : ws_reserve_naive(w, a.n, st));
   else if (a.n >= 2) NB_TRY(ws_reserve(w, a.n, a.key_bits));
   if (pm) NB_CUDA(cudaEventRecord(pm->start, st));
   if (force == NB_FORCE_BH && a.n < 2) {
@@ -555,7 +566,7 @@ static int sim_capture(nb_sim* s) {
   if (resolve_force(s->p, s->n) == NB_FORCE_BH)
     NB_TRY(ws_reserve(s->ws, s->n, s->p.key_bits));
   else
-    NB_TRY(ws_reserve_naive(s->ws, s->n));
+    NB_TRY(ws_reserve_naive(s->ws, s->n, s->stream));
   cudaGraph_t g = nullptr;
   NB_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   int rc = sim_step_eager(s, nullptr);
@@ -667,7 +678,7 @@ int nb_sim_create(int n, const float* pos4, const float* vel4,
     if ((rc = ws_basic(s->ws)) != NB_OK) break;
     // the force module's workspace now, not inside the first (timed) call
     if (resolve_force(s->p, n) == NB_FORCE_NAIVE)
-      rc = ws_reserve_naive(s->ws, n);
+      rc = ws_reserve_naive(s->ws, n, s->stream);
     else if (n >= 2)
       rc = ws_reserve(s->ws, n, s->p.key_bits);
     if (rc != NB_OK) break;

@@ -136,6 +136,7 @@ struct Workspace {
   int part_cap = 0;               // elements
   unsigned* tickets = nullptr;    // per i-tile tickets
   int tickets_cap = 0;
+  int ap_n = 0;                   // largest n whose all-pairs scratch was reserved
   // energy
   double* epart = nullptr;        // per-block partials [blocks][6]
   int epart_cap = 0;
@@ -157,8 +158,8 @@ constexpr int kPrepMaxBlocks = 1024;
 int ws_reserve(Workspace& w, int n, int key_bits);
 struct APGeom;
 int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g);
-// all-pairs scratch of the kernel that n particles use
-int ws_reserve_naive(Workspace& w, int n);
+// all-pairs scratch of the kernel that n particles use on `st`
+int ws_reserve_naive(Workspace& w, int n, cudaStream_t st);
 int ws_reserve_energy(Workspace& w, int blocks, int parts);
 void ws_free(Workspace& w);
 
@@ -264,15 +265,18 @@ __device__ __forceinline__ void chain_wait() {
 __device__ __forceinline__ void chain_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// Adds the attribute to a launch of the chain (room for one more in `at`).
-inline void chained_attribute(cudaStream_t st, cudaLaunchConfig_t* cfg,
-                              cudaLaunchAttribute* at) {
+inline bool is_capturing(cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
     cudaGetLastError();
-    cs = cudaStreamCaptureStatusNone;
+    return false;
   }
-  if (cs != cudaStreamCaptureStatusNone) return;
+  return cs != cudaStreamCaptureStatusNone;
+}
+// Adds the attribute to a launch of the chain (room for one more in `at`).
+inline void chained_attribute(cudaStream_t st, cudaLaunchConfig_t* cfg,
+                              cudaLaunchAttribute* at) {
+  if (is_capturing(st)) return;
   at[cfg->numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[cfg->numAttrs].val.programmaticStreamSerializationAllowed = 1;
   ++cfg->numAttrs;
