@@ -111,6 +111,7 @@ static int ws_basic(Workspace& w) {
   NB_TRY(dalloc(&w.bbox_part, (size_t)kPrepMaxBlocks * 6));
   NB_TRY(dalloc(&w.bbox_ticket, 4));
   NB_CUDA(cudaMemset(w.bbox_ticket, 0, 4 * sizeof(unsigned)));
+  NB_TRY(dalloc(&w.pos_copy, kSymMin));
   NB_TRY(dalloc(&w.eout, 8));
   NB_TRY(dalloc(&w.eticket, 4));
   NB_CUDA(cudaMemset(w.eticket, 0, 4 * sizeof(unsigned)));
@@ -198,7 +199,6 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
     w.src_cap = npad;
   }
   size_t need = g.jsplit > 1 ? (size_t)g.jsplit * n : 1;
-  if (allpairs_sym(n)) need = std::max(need, allpairs_sym_least_f4(n));
   if (need > (size_t)w.part_cap) {
     NB_TRY(dalloc(&w.part, need));
     w.part_cap = (int)need;
@@ -240,7 +240,7 @@ void ws_free(Workspace& w) {
   cudaFree(w.bbox); cudaFree(w.bbox_part); cudaFree(w.bbox_ticket);
   cudaFree(w.src); cudaFree(w.part); cudaFree(w.tickets); cudaFree(w.epart);
   cudaFree(w.ephi); cudaFree(w.eout); cudaFree(w.eticket); cudaFree(w.counts);
-  cudaFree(w.err);
+  cudaFree(w.err); cudaFree(w.pos_copy);
   if (w.h_eout) cudaFreeHost(w.h_eout);
   if (w.h_err) cudaFreeHost(w.h_err);
   w = Workspace{};
@@ -328,9 +328,7 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   if (force == NB_FORCE_AUTO)
     force = resolve_force_tuned(force, a.n, std::sqrt(a.theta2), a.traverse);
   // workspace growth (allocation, host side) stays outside the timed region
-  if (force == NB_FORCE_NAIVE)
-    NB_TRY(allpairs_packed(a) ? ws_reserve_allpairs(w, a.n, allpairs_geometry(a.n))
-                              : ws_reserve_naive(w, a.n, st));
+  if (force == NB_FORCE_NAIVE) NB_TRY(ws_reserve_naive(w, a.n, st));
   else if (a.n >= 2) NB_TRY(ws_reserve(w, a.n, a.key_bits));
   if (pm) NB_CUDA(cudaEventRecord(pm->start, st));
   if (force == NB_FORCE_BH && a.n < 2) {
@@ -341,7 +339,7 @@ int enqueue_forces(Workspace& w, const StepArgs& a, int force, cudaStream_t st,
   }
   if (force == NB_FORCE_NAIVE) {
     // most calls' kernels read the positions themselves: nothing to pack
-    const bool pack = allpairs_packed(a);
+    const bool pack = a.n > kSymMax;
     if (pack || a.kick_drift) NB_TRY(launch_prep(w, a, false, pack, st));
     if (a.after_prep) NB_CUDA(cudaEventRecord(a.after_prep, st));
     NB_TRY(mark(pm, NB_PHASE_PREP, st));

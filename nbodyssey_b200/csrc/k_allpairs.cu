@@ -332,18 +332,30 @@ int launch_allpairs_geom(Workspace& w, const StepArgs& s, const APGeom& g,
   return NB_OK;
 }
 
-// Above kSymMax, and for forces written over the positions themselves: the
-// tiled kernel reads its sources from the packed copy, and a tile's targets
-// before any of its forces is written; the other kernels read all positions
-// to the end.
-bool allpairs_packed(const StepArgs& s) { return s.n > kSymMax || s.acc == s.pos; }
-
+// Above kSymMax the tiled kernel reads its sources from the packed copy, and a
+// tile's targets before any of its forces is written; the other kernels read
+// all positions to the end, so for forces over the positions themselves they
+// read a copy: the small kernel one of its own, the pairs-once kernel one at the
+// end of its table (nothing to allocate that a call beside them had not).
 int launch_allpairs(Workspace& w, const StepArgs& s, cudaStream_t st) {
-  if (allpairs_packed(s)) return launch_allpairs_geom(w, s, allpairs_geometry(s.n), st);
+  if (s.n > kSymMax) return launch_allpairs_geom(w, s, allpairs_geometry(s.n), st);
+  const float4* pos = s.pos;
+  size_t table = (size_t)w.part_cap;
+  if (s.acc == s.pos) {
+    float4* copy = w.pos_copy;
+    if (s.n >= kSymMin) {
+      if (table < s.n + allpairs_sym_least_f4(s.n))
+        return set_error(NB_ERR_NOMEM, "all-pairs scratch too small");
+      table -= s.n;
+      copy = w.part + table;
+    }
+    NB_CUDA(cudaMemcpyAsync(copy, s.pos, sizeof(float4) * s.n, cudaMemcpyDeviceToDevice, st));
+    pos = copy;
+  }
   if (s.n < kSymMin) {
     APArgs a{};
     a.n = s.n;
-    a.pos = s.pos;
+    a.pos = pos;
     a.eps2 = s.eps2;
     a.G = s.G;
     a.half_dt = s.half_dt;
@@ -351,8 +363,8 @@ int launch_allpairs(Workspace& w, const StepArgs& s, cudaStream_t st) {
     a.vel = s.kick_after ? s.vel : nullptr;
     return launch_allpairs_small(a, st);
   }
-  return launch_allpairs_sym(s.n, s.pos, s.acc, s.kick_after ? s.vel : nullptr, s.eps2, s.G,
-                             s.half_dt, w.part, (size_t)w.part_cap, st);
+  return launch_allpairs_sym(s.n, pos, s.acc, s.kick_after ? s.vel : nullptr, s.eps2, s.G,
+                             s.half_dt, w.part, table, st);
 }
 
 // ---------------------------------------------------------------------------

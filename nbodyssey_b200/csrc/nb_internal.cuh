@@ -137,6 +137,7 @@ struct Workspace {
   unsigned* tickets = nullptr;    // per i-tile tickets
   int tickets_cap = 0;
   int ap_n = 0;                   // largest n whose all-pairs scratch was reserved
+  float4* pos_copy = nullptr;     // [kSymMin] for forces over the positions
   // energy
   double* epart = nullptr;        // per-block partials [blocks][6]
   int epart_cap = 0;
@@ -208,7 +209,6 @@ int launch_walk(Workspace& w, const StepArgs& a, cudaStream_t st);
 // permutation of the workspace's last tree, or the identity without one
 int launch_gather_part(Workspace& w, const StepArgs& a, const float4* sorted,
                        bool use_perm, cudaStream_t st);
-bool allpairs_packed(const StepArgs& a);   // sources from the packed copy
 int launch_allpairs(Workspace& w, const StepArgs& a, cudaStream_t st);
 // energy: {E, KE, PE, Px, Py, Pz} into w.eout (device); positions hi (+lo
 // for the kinetic part is not needed).

@@ -78,3 +78,18 @@ def test_capture_of_a_larger_call_than_the_warm_up_is_refused():
         assert np.array_equal(acc.cpu().numpy(), ref)
     finally:
         dev.close()
+
+
+@pytest.mark.parametrize("n", [1, 1000, 2559, 2560, 9000, 60_001])
+def test_capture_of_forces_over_the_positions_after_a_warm_up_beside_them(n):
+    import torch
+    dev = _Dev()
+    try:
+        pos = torch.from_numpy(ic.two_disks(max(n, 2), seed=3)[0][:n]).cuda()
+        acc = torch.zeros_like(pos)
+        dev.forces(pos, acc)
+        buf = pos.clone()
+        _captured(lambda: dev.forces(buf, buf))
+        assert np.array_equal(buf.cpu().numpy(), acc.cpu().numpy())
+    finally:
+        dev.close()
