@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -124,6 +125,8 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   if (n <= w.cap && key_bits <= w.key_bits) return NB_OK;
   int cap = n > w.cap ? n : w.cap;
   int kb = key_bits > w.key_bits ? key_bits : w.key_bits;
+  w.cap = 0;   // until every array is there
+  ++w.moves;
   size_t ksz = kb == 63 ? 8 : 4;
   size_t ni = cap > 1 ? (size_t)cap - 1 : 1;
   void* k0 = w.keys;
@@ -164,28 +167,55 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   return NB_OK;
 }
 
-// Scratch of the pairs-once kernel: all rows of tiles up to 1 GiB, fewer when
-// that cannot be had (one row at least).  The whole table does not grow with n
-// throughout (a larger tile makes it smaller), and a capture cannot allocate:
-// there a size that a larger call has reserved for takes the table at hand, in
-// passes over what it holds.
+size_t allpairs_table_limit_f4() {
+  const char* e = std::getenv("NBODY_B200_ALLPAIRS_MIB");
+  if (!e || !*e) return ~(size_t)0;
+  return (size_t)std::strtoull(e, nullptr, 10) << 16;
+}
+
+// Grows an array of a workspace.  The capacity is 0 while there is none, so a
+// failed growth leaves nothing that a smaller call could take for room.
+template <typename T>
+static int regrow(T** p, int* cap, size_t count) {
+  *cap = 0;
+  NB_TRY(dalloc(p, count));
+  *cap = (int)count;
+  return NB_OK;
+}
+
+// Scratch of the pairs-once kernel: all rows of tiles up to 1 GiB, half as much
+// again and again when that cannot be had, down to a copy of the positions and
+// a pass's least.  A size that could not be had is not asked for a second time,
+// so calls that follow find their table and neither free nor allocate.
+// The whole table does not grow with n throughout (a larger tile makes it
+// smaller), and a capture cannot allocate: there a size that a larger call has
+// reserved for takes the table at hand, in passes over what it holds.
 static int ws_reserve_allpairs_sym(Workspace& w, int n, cudaStream_t st) {
   NB_TRY(ws_basic(w));
   const size_t row = allpairs_sym_row_f4(n);
   const size_t tiles = allpairs_sym_geometry(n).tiles;
-  size_t rows = std::max<size_t>(1, std::min(tiles, ((size_t)1 << 26) / row));
-  if ((size_t)w.part_cap < rows * row) {
-    if (n <= w.ap_n && is_capturing(st)) return NB_OK;
-    for (;; rows = (rows + 1) / 2) {
-      w.part_cap = 0;
-      const int rc = dalloc(&w.part, rows * row);
+  const size_t want = row * std::max<size_t>(1, std::min(tiles, kSymTableMax / row));
+  const size_t least = n + allpairs_sym_least_f4(n);
+  const size_t have = (size_t)w.part_cap;
+  if (have < want && (have < least || want < w.part_refused)) {
+    if (is_capturing(st)) {
+      if (n <= w.ap_n) return NB_OK;
+      return set_error(NB_ERR_NOMEM, "all-pairs scratch cannot grow under stream capture");
+    }
+    ++w.moves;
+    for (size_t f4 = want;; f4 = std::max(least, f4 / 2)) {
+      int rc = NB_ERR_NOMEM;
+      if (f4 > least && f4 > allpairs_table_limit_f4())
+        set_error(rc, "all-pairs table above NBODY_B200_ALLPAIRS_MIB");
+      else
+        rc = regrow(&w.part, &w.part_cap, f4);
       if (rc == NB_OK) break;
-      if (rows == 1) {
+      w.part_refused = std::min(w.part_refused, f4);
+      if (f4 == least) {
         w.ap_n = 0;
         return rc;
       }
     }
-    w.part_cap = (int)(rows * row);
   }
   w.ap_n = std::max(w.ap_n, n);
   return NB_OK;
@@ -195,21 +225,22 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
   NB_TRY(ws_basic(w));
   int npad = (n + kSrcTile - 1) / kSrcTile * kSrcTile;
   if (npad > w.src_cap) {
-    NB_TRY(dalloc(&w.src, (size_t)npad));   // 2 float4 per pair = npad float4
-    w.src_cap = npad;
+    ++w.moves;
+    NB_TRY(regrow(&w.src, &w.src_cap, (size_t)npad));   // 2 float4 per pair = npad float4
   }
   size_t need = g.jsplit > 1 ? (size_t)g.jsplit * n : 1;
   if (need > (size_t)w.part_cap) {
-    NB_TRY(dalloc(&w.part, need));
-    w.part_cap = (int)need;
+    ++w.moves;
+    w.ap_n = 0;
+    NB_TRY(regrow(&w.part, &w.part_cap, need));
   }
   int itiles = g.itiles + 1;
   if (itiles > w.tickets_cap) {
-    NB_TRY(dalloc(&w.tickets, (size_t)itiles));
+    ++w.moves;
+    NB_TRY(regrow(&w.tickets, &w.tickets_cap, (size_t)itiles));
     NB_CUDA(cudaMemset(w.tickets, 0, itiles * sizeof(unsigned)));
-    w.tickets_cap = itiles;
   }
-  if ((size_t)w.part_cap >= allpairs_sym_least_f4(n)) w.ap_n = std::max(w.ap_n, n);
+  if ((size_t)w.part_cap >= n + allpairs_sym_least_f4(n)) w.ap_n = std::max(w.ap_n, n);
   return NB_OK;
 }
 
@@ -221,14 +252,8 @@ int ws_reserve_naive(Workspace& w, int n, cudaStream_t st) {
 
 int ws_reserve_energy(Workspace& w, int blocks, int parts) {
   NB_TRY(ws_basic(w));
-  if (blocks * 5 > w.epart_cap) {
-    NB_TRY(dalloc(&w.epart, (size_t)blocks * 5));
-    w.epart_cap = blocks * 5;
-  }
-  if (parts > w.ephi_cap) {
-    NB_TRY(dalloc(&w.ephi, (size_t)parts));
-    w.ephi_cap = parts;
-  }
+  if (blocks * 5 > w.epart_cap) NB_TRY(regrow(&w.epart, &w.epart_cap, (size_t)blocks * 5));
+  if (parts > w.ephi_cap) NB_TRY(regrow(&w.ephi, &w.ephi_cap, (size_t)parts));
   return NB_OK;
 }
 
@@ -420,6 +445,7 @@ struct nb_sim {
   bool use_graphs = true;
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
+  unsigned graph_moves = 0;   // ws.moves at the capture
   // timing
   bool timing = false;
   std::vector<PhaseMarks*> pending;
@@ -582,6 +608,7 @@ static int sim_capture(nb_sim* s) {
     return set_error(NB_ERR_CUDA, std::string("cudaGraphInstantiate: ") +
                                       cudaGetErrorString(e));
   s->graph_valid = true;
+  s->graph_moves = s->ws.moves;
   return NB_OK;
 }
 
@@ -887,7 +914,8 @@ int nb_step(nb_sim* s, int nsteps) {
       continue;
     }
     if (s->use_graphs) {
-      if (!s->graph_valid) NB_TRY(sim_capture(s));
+      // a graph holds the addresses of the scratch it was captured with
+      if (!s->graph_valid || s->graph_moves != s->ws.moves) NB_TRY(sim_capture(s));
       NB_CUDA(cudaGraphLaunch(s->graph, s->stream));
     } else {
       NB_TRY(sim_step_eager(s, nullptr));

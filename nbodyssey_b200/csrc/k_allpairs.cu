@@ -428,7 +428,7 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
   for (int s = 0; s < nsims; ++s)
     if (sims[s].active && sims[s].force == NB_FORCE_NAIVE) whole += ap_region_whole_f4(sims[s].n);
   auto size_of = [&](int n) {
-    return whole <= ((size_t)1 << 26) ? ap_region_whole_f4(n) : ap_region_f4(n);
+    return whole <= kSymTableMax ? ap_region_whole_f4(n) : ap_region_f4(n);
   };
   struct Pending { int a; APGeom g; };
   std::vector<Pending> todo;

@@ -137,7 +137,10 @@ struct Workspace {
   unsigned* tickets = nullptr;    // per i-tile tickets
   int tickets_cap = 0;
   int ap_n = 0;                   // largest n whose all-pairs scratch was reserved
+  size_t part_refused = ~(size_t)0;   // smallest all-pairs table that could not be had
   float4* pos_copy = nullptr;     // [kSymMin] for forces over the positions
+  // counts the moves of any array that a captured step uses
+  unsigned moves = 0;
   // energy
   double* epart = nullptr;        // per-block partials [blocks][6]
   int epart_cap = 0;
@@ -368,6 +371,10 @@ struct SymGeom {
   int tiles, chunks;
 };
 SymGeom allpairs_sym_geometry(int n);
+constexpr size_t kSymTableMax = (size_t)1 << 26;   // float4 of a table: 1 GiB
+// NBODY_B200_ALLPAIRS_MIB in float4: larger tables count as not to be had (no
+// limit without it)
+size_t allpairs_table_limit_f4();
 // scratch float4 of one row of tiles, and the least a pass runs with; any
 // amount from that on gives the same bits
 size_t allpairs_sym_row_f4(int n);

@@ -1,5 +1,5 @@
 """All-pairs scratch: calls under stream capture on a workspace that has been
-used before."""
+used before, tables that cannot be had, and captured steps whose scratch moves."""
 import ctypes
 
 import numpy as np
@@ -93,3 +93,82 @@ def test_capture_of_forces_over_the_positions_after_a_warm_up_beside_them(n):
         assert np.array_equal(buf.cpu().numpy(), acc.cpu().numpy())
     finally:
         dev.close()
+
+
+# rows of tiles at a time (8 MiB) and chunks of one row (1 MiB) of a table of 38
+@pytest.mark.parametrize("mib", ["8", "1"])
+def test_table_that_cannot_be_had(monkeypatch, mib):
+    """A table refused (here by the limit) is done without: the same bits from a
+    smaller one, eagerly, through the step graph and under capture, and nothing
+    changes for the handle once there is room again."""
+    import torch
+    n = 20_001
+    pos, vel = ic.two_disks(n, seed=4)
+    with api.Simulation(pos, vel, PRM) as sim:
+        ref = sim.compute_forces()
+        sim.step(3)
+        end = sim.positions()
+    monkeypatch.setenv("NBODY_B200_ALLPAIRS_MIB", mib)
+    with api.Simulation(pos, vel, PRM) as sim:
+        for _ in range(2):
+            assert np.array_equal(sim.compute_forces(), ref)
+        sim.step(1)
+        sim.compute_forces()
+        sim.step(1)
+        monkeypatch.delenv("NBODY_B200_ALLPAIRS_MIB")
+        sim.compute_forces()
+        sim.step(1)
+        assert np.array_equal(sim.positions(), end)
+    monkeypatch.setenv("NBODY_B200_ALLPAIRS_MIB", mib)
+    dev = _Dev()
+    try:
+        d_pos = torch.from_numpy(pos).cuda()
+        acc = torch.zeros_like(d_pos)
+        dev.forces(d_pos, acc)
+        acc.zero_()
+        _captured(lambda: dev.forces(d_pos, acc))
+        assert np.array_equal(acc.cpu().numpy(), ref)
+        buf = d_pos.clone()
+        dev.forces(buf, buf)   # the copy of the positions beside such a table
+        assert np.array_equal(buf.cpu().numpy(), ref)
+    finally:
+        dev.close()
+
+
+def test_limit_bounds_the_memory_of_a_handle(monkeypatch):
+    """Without it 262,144 particles take 0.8 GB."""
+    import torch
+    pos, vel = ic.two_disks(262_144, seed=5)
+    with api.Simulation(pos[:64].copy(), vel[:64].copy(), PRM):   # kernels and tuning first
+        pass
+    monkeypatch.setenv("NBODY_B200_ALLPAIRS_MIB", "64")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    with api.Simulation(pos, vel, PRM):
+        assert free - torch.cuda.mem_get_info()[0] < 160 << 20
+
+
+def test_step_graph_follows_scratch_that_moved():
+    """Above 2^20 particles a table set by hand can ask for more partials: a
+    force call then moves the scratch that the captured step uses."""
+    n = (1 << 20) + 1
+    pos, vel = ic.two_disks(n, seed=6)
+    base = api.tune_get()
+    out = []
+    try:
+        for graphs in (True, False):
+            api.tune_set(dict(base, ap_threads=[256] * L.NB_TUNE_BUCKETS,
+                              ap_k=[8] * L.NB_TUNE_BUCKETS,
+                              ap_ctas=[1024] * L.NB_TUNE_BUCKETS))   # 513 tiles: 2 chunks
+            with api.Simulation(pos, vel, PRM) as sim:
+                sim.set_graphs(graphs)
+                sim.step(1)
+                api.tune_set(dict(base, ap_threads=[256] * L.NB_TUNE_BUCKETS,
+                                  ap_k=[8] * L.NB_TUNE_BUCKETS,
+                                  ap_ctas=[3000] * L.NB_TUNE_BUCKETS))   # 6 chunks
+                sim.compute_forces()
+                sim.step(1)
+                out.append(sim.positions())
+    finally:
+        api.tune_set(base)
+    assert np.array_equal(*out)
