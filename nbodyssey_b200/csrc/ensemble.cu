@@ -178,28 +178,9 @@ int ens_device_error(nb_ensemble* h) {
   return NB_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-int nb_ensemble_create(int nsims, const int* n, const float* pos4,
-                       const float* vel4, const nb_params* params,
-                       nb_ensemble** out) {
-  if (!out) return set_error(NB_ERR_INVALID, "out is NULL");
-  *out = nullptr;
-  if (nsims <= 0 || nsims > kEnsMaxSims)
-    return set_error(NB_ERR_INVALID, "nsims must be in [1, " + std::to_string(kEnsMaxSims) + "]");
-  if (!n || !pos4 || !vel4 || !params) return set_error(NB_ERR_INVALID, "NULL argument");
-  long long slots = 0, total = 0;
-  for (int s = 0; s < nsims; ++s) {
-    if (n[s] <= 0) return set_error(NB_ERR_INVALID, "every n must be > 0");
-    NB_TRY(ens_check_params(params[s]));
-    slots += (n[s] + 31) / 32 * 32;
-    total += n[s];
-  }
-  if (slots >= (1ll << 29)) return set_error(NB_ERR_INVALID, "too many particles in total");
-  NB_TRY(warm_kernels());         // first use on this device: load the kernels
-  NB_TRY(tune_ensure(nullptr));   // first use on this device: the tuning table
+// With `least` the all-pairs simulations get the least regions they run with.
+int ens_create(int nsims, const int* n, const float* pos4, const float* vel4,
+               const nb_params* params, bool least, nb_ensemble** out) {
   nb_ensemble* h = new nb_ensemble();
   h->nsims = nsims;
   h->n.assign(n, n + nsims);
@@ -276,9 +257,13 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
     }
     if (rc != NB_OK) break;
     if ((rc = ens_alloc(h, &e.walk_ctr, 2)) != NB_OK) break;
-    h->ap_pool_f4 = plan_ens_allpairs(sims.data(), nsims, nullptr, h->ap);
+    h->ap_pool_f4 = plan_ens_allpairs(sims.data(), nsims, nullptr, h->ap, nullptr, nullptr, least);
     if (h->ap_pool_f4 > 0) {
       EnsAllPairs& ap = h->ap;
+      if (!least && h->ap_pool_f4 > allpairs_table_limit_f4()) {
+        rc = set_error(NB_ERR_NOMEM, "all-pairs tables above NBODY_B200_ALLPAIRS_MIB");
+        break;
+      }
       if ((rc = ens_alloc(h, &ap.d_pool, h->ap_pool_f4)) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_args, ap.args.size())) != NB_OK) break;
       if ((rc = ens_alloc(h, &ap.d_items, ap.items.size())) != NB_OK) break;
@@ -350,6 +335,33 @@ int nb_ensemble_create(int nsims, const int* n, const float* pos4,
   }
   *out = h;
   return NB_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int nb_ensemble_create(int nsims, const int* n, const float* pos4,
+                       const float* vel4, const nb_params* params,
+                       nb_ensemble** out) {
+  if (!out) return set_error(NB_ERR_INVALID, "out is NULL");
+  *out = nullptr;
+  if (nsims <= 0 || nsims > kEnsMaxSims)
+    return set_error(NB_ERR_INVALID, "nsims must be in [1, " + std::to_string(kEnsMaxSims) + "]");
+  if (!n || !pos4 || !vel4 || !params) return set_error(NB_ERR_INVALID, "NULL argument");
+  long long slots = 0, total = 0;
+  for (int s = 0; s < nsims; ++s) {
+    if (n[s] <= 0) return set_error(NB_ERR_INVALID, "every n must be > 0");
+    NB_TRY(ens_check_params(params[s]));
+    slots += (n[s] + 31) / 32 * 32;
+    total += n[s];
+  }
+  if (slots >= (1ll << 29)) return set_error(NB_ERR_INVALID, "too many particles in total");
+  NB_TRY(warm_kernels());         // first use on this device: load the kernels
+  NB_TRY(tune_ensure(nullptr));   // first use on this device: the tuning table
+  // whole all-pairs tables if they can be had (1 GiB at most), else the least
+  const int rc = ens_create(nsims, n, pos4, vel4, params, false, out);
+  return rc == NB_ERR_NOMEM ? ens_create(nsims, n, pos4, vel4, params, true, out) : rc;
 }
 
 int nb_ensemble_force(const nb_ensemble* h, int sim, int* force) {

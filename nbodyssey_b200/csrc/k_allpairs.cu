@@ -413,7 +413,7 @@ size_t ap_region_whole_f4(int n) {
 }
 
 size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of,
-                         EnsAllPairs& ap, const size_t* region_cap, int* too_small) {
+                         EnsAllPairs& ap, const size_t* region_cap, int* too_small, bool least) {
   if (too_small) *too_small = 0;
   ap.args.clear();
   ap.sim.clear();
@@ -428,7 +428,7 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
   for (int s = 0; s < nsims; ++s)
     if (sims[s].active && sims[s].force == NB_FORCE_NAIVE) whole += ap_region_whole_f4(sims[s].n);
   auto size_of = [&](int n) {
-    return whole <= kSymTableMax ? ap_region_whole_f4(n) : ap_region_f4(n);
+    return whole <= kSymTableMax && !least ? ap_region_whole_f4(n) : ap_region_f4(n);
   };
   struct Pending { int a; APGeom g; };
   std::vector<Pending> todo;
@@ -448,10 +448,10 @@ size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of
     a.half_dt = d.half_dt;
     const size_t r = region_of ? region_of[s] : next;
     const size_t size = region_cap ? region_cap[s] : size_of(d.n);
-    const size_t least = allpairs_sym(d.n) ? allpairs_sym_least_f4(d.n)
-                         : d.n < kSymMin   ? 0
-                                           : ap_region_f4(d.n);
-    if (least > size) {   // the table changed
+    const size_t need = allpairs_sym(d.n) ? allpairs_sym_least_f4(d.n)
+                        : d.n < kSymMin   ? 0
+                                          : ap_region_f4(d.n);
+    if (need > size) {   // the table changed
       if (too_small) ++*too_small;
       continue;
     }

@@ -561,13 +561,13 @@ size_t ap_region_whole_f4(int n);
 // Host plan of the simulations whose SimDesc.force is NB_FORCE_NAIVE and that
 // are active: geometry, items, and the region of simulation s at
 // region_of[s] (nullptr: back to back from 0, whole tables while they sum up to
-// 1 GiB at most).  With region_cap, a simulation
+// 1 GiB at most and not `least`).  With region_cap, a simulation
 // whose geometry now needs more than region_cap[s] float4 (the tuning table
 // changed since its region was sized) is left out and counted in *too_small.
 // Returns the pool size used.
 size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of,
                          EnsAllPairs& ap, const size_t* region_cap = nullptr,
-                         int* too_small = nullptr);
+                         int* too_small = nullptr, bool least = false);
 // Points the per-simulation arguments at the batch's arrays and the pool and
 // uploads them with the items and source offsets (stream-ordered; the host
 // vectors must live until the copies ran).

@@ -7,6 +7,7 @@ import pytest
 
 from nbodyssey_b200 import _lib as L
 from nbodyssey_b200 import api, ic
+from nbodyssey_b200.ensemble import Ensemble
 
 pytestmark = pytest.mark.gpu
 EPS = 0.05
@@ -172,3 +173,32 @@ def test_step_graph_follows_scratch_that_moved():
     finally:
         api.tune_set(base)
     assert np.array_equal(*out)
+
+
+def test_batch_tables_that_cannot_be_had(monkeypatch):
+    """Eight simulations of 40,000 particles take 614 MB with whole tables; where
+    those cannot be had the batch is made with the least regions (160 MB with the
+    default shapes), its results unchanged."""
+    import ctypes as C
+
+    import torch
+    base = api.tune_get()
+    t = L.nb_tune_table()
+    L.check(L.load().nb_tune_defaults(C.byref(t)))
+    try:
+        L.check(L.load().nb_tune_set(C.byref(t)))
+        states = [ic.two_disks(40_000, seed=k) for k in range(8)]
+        with Ensemble(states, PRM) as ens:
+            ens.step(2)
+            ref = [ens.state(s) for s in range(8)]
+        monkeypatch.setenv("NBODY_B200_ALLPAIRS_MIB", "256")
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        with Ensemble(states, PRM) as ens:
+            assert free - torch.cuda.mem_get_info()[0] < 350 << 20
+            ens.step(2)
+            for s in range(8):
+                p, v = ens.state(s)
+                assert np.array_equal(p, ref[s][0]) and np.array_equal(v, ref[s][1])
+    finally:
+        api.tune_set(base)
