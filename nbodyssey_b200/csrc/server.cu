@@ -63,6 +63,7 @@ struct Request {
   int force = NB_FORCE_BH;    // the module it gets alone (AUTO resolved)
   int ap_chunk = -1;          // all-pairs: its region in the scratch pool
   int ap_len = 0;             // (units of kApChunk float4)
+  int ap_least = 0;           // the length it can run with
   int steps_done = 0;
   int frames = 0;
   bool primed = false;
@@ -96,6 +97,7 @@ struct nb_server {
   float4* d_ap_pool = nullptr;
   int ap_chunks = 0;
   std::map<int, int> ap_free;        // start chunk -> length
+  long long ap_kept = 0;             // the running requests' least lengths
   std::vector<size_t> ap_region;     // by sim id: region offset (float4)
   std::vector<size_t> ap_region_cap; // by sim id: region size (float4)
   EnsAllPairs ap;
@@ -188,12 +190,44 @@ void give_range(std::map<int, int>& fl, int start, int len) {
 
 int ap_chunks_of(int n) { return (int)((ap_region_f4(n) + kApChunk - 1) / kApChunk); }
 
-// The region a request takes: its whole table of partials when that is at most
-// 1/64 of the pool (as many requests run side by side as before), else the
-// least it can run with.
-int ap_chunks_taken(const nb_server* s, int n) {
+// Gives running request r the region of `len` units at `start`.  Packed sources
+// start with zero-mass pads, their tickets at zero; the other all-pairs kernels
+// read nothing of a region that the same step has not written.
+int ap_place(nb_server* s, Request* r, int start, int len) {
+  r->ap_chunk = start;
+  r->ap_len = len;
+  s->ap_region[r->sim] = (size_t)start * kApChunk;
+  s->ap_region_cap[r->sim] = (size_t)len * kApChunk;
+  s->table_dirty = true;
+  if (r->n > kSymMax)
+    NB_CUDA(cudaMemsetAsync(s->d_ap_pool + s->ap_region[r->sim], 0,
+                            sizeof(float4) * s->ap_region_cap[r->sim], s->stream));
+  return NB_OK;
+}
+
+// A region for a request that can run with `least` units: its whole table when
+// that is at most 1/64 of the pool and free, else the least.  Where neither is
+// free but the least would be if every running request kept only its own, they
+// move together at the front of the pool first (a region holds nothing between
+// steps, and the next step's launches follow this one's in the stream), so whole
+// tables keep nobody out.  -1 when there is no room.
+int ap_take(nb_server* s, int n, int least, int* start, int* len) {
   const size_t whole = (ap_region_whole_f4(n) + kApChunk - 1) / kApChunk;
-  return whole * 64 <= (size_t)s->ap_chunks ? (int)whole : ap_chunks_of(n);
+  *len = (int)whole;
+  *start = whole * 64 <= (size_t)s->ap_chunks ? take_range(s->ap_free, *len) : -1;
+  if (*start >= 0) return NB_OK;
+  *len = least;
+  *start = take_range(s->ap_free, *len);
+  if (*start >= 0) return NB_OK;
+  if (s->ap_kept + least > s->ap_chunks) return NB_OK;
+  for (Request* r : s->finishing) r->ap_chunk = -1;   // their last step is queued
+  s->ap_free.clear();
+  s->ap_free[0] = s->ap_chunks;
+  for (Request* r : s->running)
+    if (r->ap_chunk >= 0)
+      NB_TRY(ap_place(s, r, take_range(s->ap_free, r->ap_least), r->ap_least));
+  *start = take_range(s->ap_free, *len);
+  return NB_OK;
 }
 
 int mkdirs(const std::string& path) {
@@ -279,23 +313,17 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
     Request* r = s->waiting[k];
     const int nb32 = (r->n + 31) / 32;
     if (s->free_ids.empty()) break;
-    int ap0 = -1;
-    if (r->force == NB_FORCE_NAIVE) {
-      ap0 = take_range(s->ap_free, ap_chunks_taken(s, r->n));
-      if (ap0 < 0) { ++k; continue; }
-    }
     const int b0 = take_range(s->free_blocks, nb32);
-    if (b0 < 0) {
-      if (ap0 >= 0) give_range(s->ap_free, ap0, ap_chunks_taken(s, r->n));
-      ++k;
-      continue;
-    }
-    if (ap0 >= 0) {
-      r->ap_chunk = ap0;
-      r->ap_len = ap_chunks_taken(s, r->n);
-      // sources start with zero-mass pads and tickets at zero
-      NB_CUDA(cudaMemsetAsync(s->d_ap_pool + (size_t)ap0 * kApChunk, 0,
-                              sizeof(float4) * kApChunk * (size_t)r->ap_len, s->stream));
+    if (b0 < 0) { ++k; continue; }
+    int ap0 = -1, ap_len = 0;
+    if (r->force == NB_FORCE_NAIVE) {
+      r->ap_least = ap_chunks_of(r->n);
+      NB_TRY(ap_take(s, r->n, r->ap_least, &ap0, &ap_len));
+      if (ap0 < 0) {
+        give_range(s->free_blocks, b0, nb32);
+        ++k;
+        continue;
+      }
     }
     std::sort(s->free_ids.begin(), s->free_ids.end(), std::greater<int>());
     const int id = s->free_ids.back();
@@ -322,8 +350,11 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
     d.active = 2;   // a(x0) in the step it joins
     d.compensated = r->p.compensated ? 1 : 0;
     d.force = r->force;
-    s->ap_region[id] = r->ap_chunk >= 0 ? (size_t)r->ap_chunk * kApChunk : 0;
-    s->ap_region_cap[id] = r->ap_chunk >= 0 ? (size_t)r->ap_len * kApChunk : 0;
+    s->ap_region[id] = s->ap_region_cap[id] = 0;
+    if (ap0 >= 0) {
+      NB_TRY(ap_place(s, r, ap0, ap_len));
+      s->ap_kept += r->ap_least;
+    }
     for (int b = 0; b < nb32; ++b) s->blk[b0 + b] = id;
     s->table_dirty = true;
     s->running.push_back(r);
@@ -459,6 +490,7 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
                             cudaMemcpyDeviceToHost, s->stream));
     NB_CUDA(cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming));
     NB_CUDA(cudaEventRecord(r->done_ev, s->stream));
+    if (r->ap_chunk >= 0) s->ap_kept -= r->ap_least;
     s->finishing.push_back(r);
     s->running.erase(s->running.begin() + k);
   }

@@ -1,5 +1,7 @@
-"""The server's all-pairs scratch pool: what is admitted follows from
-the least region a request can run with."""
+"""The server's all-pairs scratch pool: what is admitted and what runs
+side by side follow from the least region a request can run with."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -40,3 +42,27 @@ def test_a_region_smaller_than_one_row_of_tiles(table, n):
         p, v = srv.result(rid)
     q, w = _alone(pos, vel, 3)
     assert np.array_equal(p, q) and np.array_equal(v, w)
+
+
+def test_whole_tables_do_not_keep_requests_out(table):
+    """150 requests of 2,560 particles: their least regions (16 units of 16 KiB
+    with the default shapes) fit the pool of 3,200 units, their whole tables (50)
+    do not."""
+    t = L.nb_tune_table()
+    L.check(L.load().nb_tune_defaults(ctypes.byref(t)))
+    table["ap_threads"], table["ap_k"] = list(t.ap_threads), list(t.ap_k)
+    table["ap_ctas"] = list(t.ap_ctas)
+    api.tune_set(table)
+    states = [ic.two_disks(2560, seed=k) for k in range(4)]
+    steps = 2500
+    with Server(hbm_budget_bytes=3200 * 16384 * 8, max_sims=256) as srv:
+        ids = [srv.submit(*states[k % 4], PRM, steps) for k in range(150)]
+        for rid in ids:
+            srv.wait(rid, 120)
+        peak = srv.stats()["peak_running"]
+        got = [srv.result(rid) for rid in ids]
+    assert peak == 150
+    for k, (pos, vel) in enumerate(states):
+        q, w = _alone(pos, vel, steps)
+        for p, v in got[k::4]:
+            assert np.array_equal(p, q) and np.array_equal(v, w)
