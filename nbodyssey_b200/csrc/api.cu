@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "build_geometry.h"
 #include "nb_internal.cuh"
 
 namespace nb {
@@ -142,10 +143,6 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   NB_TRY(dalloc(&w.nodes, ni));
   NB_TRY(dalloc(&w.pairs, (size_t)cap));
   NB_TRY(dalloc(&w.parent, 2 * (size_t)cap));
-  for (int i = 0; i < 2; ++i) {
-    NB_TRY(dalloc(&w.seg[i], build_seg_entries(cap)));
-    NB_TRY(dalloc(&w.seg_count[i], build_groups(cap)));
-  }
   NB_TRY(dalloc(&w.sums, ni));
   NB_TRY(dalloc(&w.box_lo, ni));
   NB_TRY(dalloc(&w.box_hi, ni));
@@ -158,7 +155,16 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   NB_CUDA(cudaMemset(w.pairs, 0, (size_t)cap * sizeof(PairRec)));
   w.status_tiles = sort_status_tiles(cap);
   size_t words = 8 * kSortRadix + 8 + (size_t)8 * w.status_tiles * kSortRadix;
-  NB_TRY(dalloc(&w.hist, words));
+  // the sort's words and the build's segments in one allocation: each takes about
+  // 0.3 ms of a first call from 1 MB on, whatever its size
+  static_assert(kSortRadix % 2 == 0, "the segments are 8-byte aligned");
+  const size_t segs = build_seg_entries(cap, kb), groups = build_groups(cap, kb);
+  NB_TRY(dalloc(&w.hist, words + 4 * (segs + groups)));
+  int2* at = reinterpret_cast<int2*>(w.hist + words);
+  for (int i = 0; i < 2; ++i, at += segs + groups) {
+    w.seg[i] = at;
+    w.seg_count[i] = at + segs;
+  }
   NB_CUDA(cudaMemset(w.hist, 0, words * sizeof(uint32_t)));
   w.tile_ctr = w.hist + 8 * kSortRadix;
   w.status = w.hist + 8 * kSortRadix + 8;
@@ -260,7 +266,6 @@ int ws_reserve_energy(Workspace& w, int blocks, int parts) {
 void ws_free(Workspace& w) {
   cudaFree(w.keys); cudaFree(w.keys_alt); cudaFree(w.vals); cudaFree(w.vals_alt);
   cudaFree(w.pos_sorted); cudaFree(w.nodes); cudaFree(w.pairs); cudaFree(w.parent);
-  for (int i = 0; i < 2; ++i) { cudaFree(w.seg[i]); cudaFree(w.seg_count[i]); }
   cudaFree(w.sums); cudaFree(w.box_lo); cudaFree(w.box_hi); cudaFree(w.hist);
   cudaFree(w.bbox); cudaFree(w.bbox_part); cudaFree(w.bbox_ticket);
   cudaFree(w.src); cudaFree(w.part); cudaFree(w.tickets); cudaFree(w.epart);

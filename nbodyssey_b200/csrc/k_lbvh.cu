@@ -10,6 +10,7 @@
 #include <cuda/atomic>
 #include <mutex>
 
+#include "build_geometry.h"
 #include "nb_internal.cuh"
 
 namespace cg = cooperative_groups;
@@ -842,7 +843,6 @@ __device__ __forceinline__ int clz_k(uint64_t x) { return __clzll((long long)x);
 // closes the root.
 // ---------------------------------------------------------------------------
 constexpr int kLevelThreads = 512;     // later levels
-constexpr int kLevelItems = 2048;      // capacity of a later level's CTA
 constexpr int kSplitEmpty = -1;
 constexpr int kSplitDone = -2;
 // d of the missing split left of the tree's first leaf and right of its last
@@ -851,12 +851,6 @@ constexpr int kSplitDone = -2;
 constexpr int kDeltaFirst = -1;
 constexpr int kDeltaLast = -2;
 
-__host__ __device__ constexpr int level_seg(int key_bits) {
-  return key_bits == 63 ? 192 : 128;
-}
-__host__ __device__ constexpr int level_fan(int key_bits) {
-  return (kLevelItems - 1) / level_seg(key_bits);
-}
 __host__ __device__ constexpr size_t level_smem(int cap) {
   // cells (FP64 sums, box lo, box hi), meta, positions, deltas, exchange
   // words, two arrival lists, scan scratch and list counters
@@ -1389,31 +1383,6 @@ static LevelArgs level_args(Workspace& w, const StepArgs& a) {
   b.fan = level_fan(a.key_bits);
   b.err = w.err;
   return b;
-}
-
-// Launches of later levels above `groups` groups.
-static int later_levels(int groups, int fan) {
-  int lv = 0;
-  for (; groups > 1; ++lv) groups = (groups + fan - 1) / fan;
-  return lv;
-}
-
-// Leaves per CTA at the first level: the fewest that need no more levels than
-// groups of 1,024 do.  A first level lasts as long as its CTAs' climbs, which
-// grow with the group, and a later level about 10 us whatever it holds.  Both
-// levels together: 36 us against 46 at n = 20,011 (256 leaves), 46 / 48 at 100,000
-// (512), 110 / 119 at 1M (512).
-static int leaf_group(int n, int fan) {
-  const int lv = later_levels((n + 1023) / 1024, fan);
-  for (int g : {256, 512})
-    if (later_levels((n + g - 1) / g, fan) <= lv) return g;
-  return 1024;
-}
-
-size_t build_groups(int cap) { return (size_t)cap / 256 + 1; }   // the smallest groups
-
-size_t build_seg_entries(int cap) {
-  return build_groups(cap) * level_seg(63);
 }
 
 template <typename K>

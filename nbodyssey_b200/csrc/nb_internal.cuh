@@ -115,8 +115,10 @@ struct Workspace {
   Node* nodes = nullptr;          // [cap-1]
   PairRec* pairs = nullptr;       // [cap] child pairs by split + the root's
   int* parent = nullptr;          // [2cap-1]
-  int2* seg[2] = {nullptr, nullptr};      // open splits per build CTA,
-  int2* seg_count[2] = {nullptr, nullptr}; // ping-pong between levels
+  // open splits per build CTA and their counts, ping-pong between levels (they
+  // lie behind the sort scratch, in its allocation)
+  int2* seg[2] = {nullptr, nullptr};
+  int2* seg_count[2] = {nullptr, nullptr};
   double4* sums = nullptr;        // [cap-1] FP64 mass-weighted sums
   float4* box_lo = nullptr;       // [cap-1]
   float4* box_hi = nullptr;       // [cap-1]
@@ -203,8 +205,6 @@ int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st);
 // memory (on a device that can hold it); the sort scratch is not used
 bool sort_in_cluster(int n, int key_bits);
 int launch_sort_cluster(Workspace& w, const StepArgs& a, cudaStream_t st);
-size_t build_groups(int cap);       // first-level CTAs at most, for any n <= cap
-size_t build_seg_entries(int cap);
 int launch_build(Workspace& w, const StepArgs& a, cudaStream_t st);
 int launch_com(Workspace& w, const StepArgs& a, cudaStream_t st);
 int launch_walk(Workspace& w, const StepArgs& a, cudaStream_t st);
