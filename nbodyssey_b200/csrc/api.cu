@@ -191,24 +191,23 @@ static int regrow(T** p, int* cap, size_t count) {
 
 // Scratch of the pairs-once kernel: all rows of tiles up to 1 GiB, half as much
 // again and again when that cannot be had, down to a copy of the positions and
-// a pass's least.  A size that could not be had is not asked for a second time,
-// so calls that follow find their table and neither free nor allocate.
-// The whole table does not grow with n throughout (a larger tile makes it
-// smaller), and a capture cannot allocate: there a size that a larger call has
-// reserved for takes the table at hand, in passes over what it holds.
+// a pass's least.  Grown only when n grows: a smaller size takes the table at
+// hand, in passes where its own would be larger (the whole table shrinks where
+// the tile grows with n) or could not be had, so no call asks twice.
 static int ws_reserve_allpairs_sym(Workspace& w, int n, cudaStream_t st) {
   NB_TRY(ws_basic(w));
+  if (n <= w.sym_n) return NB_OK;
   const size_t row = allpairs_sym_row_f4(n);
   const size_t tiles = allpairs_sym_geometry(n).tiles;
   const size_t want = row * std::max<size_t>(1, std::min(tiles, kSymTableMax / row));
   const size_t least = n + allpairs_sym_least_f4(n);
-  const size_t have = (size_t)w.part_cap;
-  if (have < want && (have < least || want < w.part_refused)) {
-    if (is_capturing(st)) {
-      if (n <= w.ap_n) return NB_OK;
+  if ((size_t)w.part_cap < want) {
+    if (is_capturing(st)) {   // no allocation here: what a larger tiled call left
+      if (n <= w.src_cap && (size_t)w.part_cap >= least) return NB_OK;
       return set_error(NB_ERR_NOMEM, "all-pairs scratch cannot grow under stream capture");
     }
     ++w.moves;
+    w.sym_n = 0;
     for (size_t f4 = want;; f4 = std::max(least, f4 / 2)) {
       int rc = NB_ERR_NOMEM;
       if (f4 > least && f4 > allpairs_table_limit_f4())
@@ -216,14 +215,10 @@ static int ws_reserve_allpairs_sym(Workspace& w, int n, cudaStream_t st) {
       else
         rc = regrow(&w.part, &w.part_cap, f4);
       if (rc == NB_OK) break;
-      w.part_refused = std::min(w.part_refused, f4);
-      if (f4 == least) {
-        w.ap_n = 0;
-        return rc;
-      }
+      if (f4 == least) return rc;
     }
   }
-  w.ap_n = std::max(w.ap_n, n);
+  w.sym_n = n;
   return NB_OK;
 }
 
@@ -237,8 +232,10 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
   size_t need = g.jsplit > 1 ? (size_t)g.jsplit * n : 1;
   if (need > (size_t)w.part_cap) {
     ++w.moves;
-    w.ap_n = 0;
+    const int sym_n = w.sym_n;
+    w.sym_n = 0;
     NB_TRY(regrow(&w.part, &w.part_cap, need));
+    w.sym_n = sym_n;
   }
   int itiles = g.itiles + 1;
   if (itiles > w.tickets_cap) {
@@ -246,7 +243,6 @@ int ws_reserve_allpairs(Workspace& w, int n, const APGeom& g) {
     NB_TRY(regrow(&w.tickets, &w.tickets_cap, (size_t)itiles));
     NB_CUDA(cudaMemset(w.tickets, 0, itiles * sizeof(unsigned)));
   }
-  if ((size_t)w.part_cap >= n + allpairs_sym_least_f4(n)) w.ap_n = std::max(w.ap_n, n);
   return NB_OK;
 }
 

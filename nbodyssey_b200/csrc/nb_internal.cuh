@@ -138,8 +138,7 @@ struct Workspace {
   int part_cap = 0;               // elements
   unsigned* tickets = nullptr;    // per i-tile tickets
   int tickets_cap = 0;
-  int ap_n = 0;                   // largest n whose all-pairs scratch was reserved
-  size_t part_refused = ~(size_t)0;   // smallest all-pairs table that could not be had
+  int sym_n = 0;                  // largest n whose all-pairs table was reserved
   float4* pos_copy = nullptr;     // [kSymMin] for forces over the positions
   // counts the moves of any array that a captured step uses
   unsigned moves = 0;

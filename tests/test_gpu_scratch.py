@@ -62,6 +62,27 @@ def test_capture_of_a_smaller_call_than_the_warm_up(n):
         dev.close()
 
 
+@pytest.mark.parametrize("n", [16_384, 24_576, 65_536, 163_840])
+def test_scratch_grows_only_with_n(n):
+    import torch
+    dev, fresh = _Dev(), _Dev()
+    try:
+        first = torch.from_numpy(ic.two_disks(n + 1, seed=1)[0]).cuda()
+        dev.forces(first, torch.zeros_like(first))
+        pos = torch.from_numpy(ic.two_disks(n, seed=2)[0]).cuda()
+        acc, ref = torch.zeros_like(pos), torch.zeros_like(pos)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        dev.forces(pos, acc)
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] == free
+        fresh.forces(pos, ref)
+        assert torch.equal(acc, ref)
+    finally:
+        dev.close()
+        fresh.close()
+
+
 def test_capture_of_a_larger_call_than_the_warm_up_is_refused():
     """As any capture that would have to allocate; the workspace stays usable."""
     import torch
