@@ -559,10 +559,11 @@ size_t ap_region_f4(int n);
 size_t ap_region_whole_f4(int n);
 // Host plan of the simulations whose SimDesc.force is NB_FORCE_NAIVE and that
 // are active: geometry, items, and the region of simulation s at
-// region_of[s] (nullptr: back to back from 0, whole tables while they sum up to
-// 1 GiB at most and not `least`).  With region_cap, a simulation
-// whose geometry now needs more than region_cap[s] float4 (the tuning table
-// changed since its region was sized) is left out and counted in *too_small.
+// region_of[s] and region_cap[s] float4; a simulation whose geometry now needs
+// more (the tuning table changed since its region was sized) is left out and
+// counted in *too_small.  Without them the regions lie back to back from 0: whole
+// tables while they sum up to 1 GiB at most, above it shares of 1 GiB, and the
+// least that they run with where `least` is set.
 // Returns the pool size used.
 size_t plan_ens_allpairs(const SimDesc* sims, int nsims, const size_t* region_of,
                          EnsAllPairs& ap, const size_t* region_cap = nullptr,

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "nb_internal.cuh"
+#include "scratch_share.h"
 
 using namespace nb;
 
@@ -61,9 +62,9 @@ struct Request {
   int sim = -1;
   int base = -1;
   int force = NB_FORCE_BH;    // the module it gets alone (AUTO resolved)
-  int ap_chunk = -1;          // all-pairs: its region in the scratch pool
-  int ap_len = 0;             // (units of kApChunk float4)
-  int ap_least = 0;           // the length it can run with
+  size_t ap_start = 0;        // all-pairs: its region in the scratch pool
+  size_t ap_len = 0;          // (units of kApChunk float4; 0: none yet)
+  size_t ap_least = 0;        // the length it can run with, 0 without all-pairs
   int steps_done = 0;
   int frames = 0;
   bool primed = false;
@@ -95,9 +96,8 @@ struct nb_server {
   // all-pairs requests: packed sources, partials and tickets per request in
   // regions of a scratch pool, and the persistent launch's work items
   float4* d_ap_pool = nullptr;
-  int ap_chunks = 0;
-  std::map<int, int> ap_free;        // start chunk -> length
-  long long ap_kept = 0;             // the running requests' least lengths
+  size_t ap_chunks = 0;
+  size_t ap_kept = 0;                // the running requests' least lengths
   std::vector<size_t> ap_region;     // by sim id: region offset (float4)
   std::vector<size_t> ap_region_cap; // by sim id: region size (float4)
   EnsAllPairs ap;
@@ -188,45 +188,38 @@ void give_range(std::map<int, int>& fl, int start, int len) {
   }
 }
 
-int ap_chunks_of(int n) { return (int)((ap_region_f4(n) + kApChunk - 1) / kApChunk); }
+size_t ap_chunks_of(size_t f4) { return (f4 + kApChunk - 1) / kApChunk; }
 
-// Gives running request r the region of `len` units at `start`.  Packed sources
-// start with zero-mass pads, their tickets at zero; the other all-pairs kernels
-// read nothing of a region that the same step has not written.
-int ap_place(nb_server* s, Request* r, int start, int len) {
-  r->ap_chunk = start;
-  r->ap_len = len;
-  s->ap_region[r->sim] = (size_t)start * kApChunk;
-  s->ap_region_cap[r->sim] = (size_t)len * kApChunk;
-  s->table_dirty = true;
-  if (r->n > kSymMax)
-    NB_CUDA(cudaMemsetAsync(s->d_ap_pool + s->ap_region[r->sim], 0,
-                            sizeof(float4) * s->ap_region_cap[r->sim], s->stream));
-  return NB_OK;
-}
-
-// A region for a request that can run with `least` units: its whole table when
-// that is at most 1/64 of the pool and free, else the least.  Where neither is
-// free but the least would be if every running request kept only its own, they
-// move together at the front of the pool first (a region holds nothing between
-// steps, and the next step's launches follow this one's in the stream), so whole
-// tables keep nobody out.  -1 when there is no room.
-int ap_take(nb_server* s, int n, int least, int* start, int* len) {
-  const size_t whole = (ap_region_whole_f4(n) + kApChunk - 1) / kApChunk;
-  *len = (int)whole;
-  *start = whole * 64 <= (size_t)s->ap_chunks ? take_range(s->ap_free, *len) : -1;
-  if (*start >= 0) return NB_OK;
-  *len = least;
-  *start = take_range(s->ap_free, *len);
-  if (*start >= 0) return NB_OK;
-  if (s->ap_kept + least > s->ap_chunks) return NB_OK;
-  for (Request* r : s->finishing) r->ap_chunk = -1;   // their last step is queued
-  s->ap_free.clear();
-  s->ap_free[0] = s->ap_chunks;
-  for (Request* r : s->running)
-    if (r->ap_chunk >= 0)
-      NB_TRY(ap_place(s, r, take_range(s->ap_free, r->ap_least), r->ap_least));
-  *start = take_range(s->ap_free, *len);
+// Lays the running all-pairs requests' regions out over the pool: whole tables
+// where they fit, else shares of it (a request alone has all of it, and of any
+// number whose least regions fit, none waits).  A region holds nothing between
+// steps, and the next step's launches follow the last one's in the stream, so
+// they may all move; packed sources, which come first and so move seldom, start
+// with zero-mass pads and their tickets at zero.  300,001 particles alone
+// in 1 GiB, default shapes: 28 ms a step, 55 with the least region.
+int ap_layout(nb_server* s) {
+  std::vector<Request*> rs;
+  for (const bool packed : {true, false})
+    for (Request* r : s->running)
+      if (r->ap_least > 0 && (r->n > kSymMax) == packed) rs.push_back(r);
+  std::vector<size_t> least, whole;
+  for (const Request* r : rs) {
+    least.push_back(r->ap_least);
+    whole.push_back(std::max(r->ap_least, ap_chunks_of(ap_region_whole_f4(r->n))));
+  }
+  const std::vector<size_t> len = share_scratch(least, whole, s->ap_chunks);
+  size_t at = 0;
+  for (size_t i = 0; i < rs.size(); at += len[i++]) {
+    Request* r = rs[i];
+    const bool same = r->ap_start == at && r->ap_len == len[i];
+    r->ap_start = at;
+    r->ap_len = len[i];
+    s->ap_region[r->sim] = at * kApChunk;
+    s->ap_region_cap[r->sim] = len[i] * kApChunk;
+    if (r->n > kSymMax && !same)
+      NB_CUDA(cudaMemsetAsync(s->d_ap_pool + s->ap_region[r->sim], 0,
+                              sizeof(float4) * s->ap_region_cap[r->sim], s->stream));
+  }
   return NB_OK;
 }
 
@@ -296,10 +289,6 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
     const int nb32 = (r->n + 31) / 32;
     for (int b = 0; b < nb32; ++b) s->blk[r->base / 32 + b] = -1;
     give_range(s->free_blocks, r->base / 32, nb32);
-    if (r->ap_chunk >= 0) {
-      give_range(s->ap_free, r->ap_chunk, r->ap_len);
-      r->ap_chunk = -1;
-    }
     s->free_ids.push_back(r->sim);
     s->table_dirty = true;
     r->state = 2;
@@ -313,18 +302,13 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
     Request* r = s->waiting[k];
     const int nb32 = (r->n + 31) / 32;
     if (s->free_ids.empty()) break;
+    const size_t least = r->force == NB_FORCE_NAIVE ? ap_chunks_of(ap_region_f4(r->n)) : 0;
+    if (s->ap_kept + least > s->ap_chunks) { ++k; continue; }
     const int b0 = take_range(s->free_blocks, nb32);
     if (b0 < 0) { ++k; continue; }
-    int ap0 = -1, ap_len = 0;
-    if (r->force == NB_FORCE_NAIVE) {
-      r->ap_least = ap_chunks_of(r->n);
-      NB_TRY(ap_take(s, r->n, r->ap_least, &ap0, &ap_len));
-      if (ap0 < 0) {
-        give_range(s->free_blocks, b0, nb32);
-        ++k;
-        continue;
-      }
-    }
+    r->ap_least = least;
+    r->ap_len = 0;
+    s->ap_kept += least;
     std::sort(s->free_ids.begin(), s->free_ids.end(), std::greater<int>());
     const int id = s->free_ids.back();
     s->free_ids.pop_back();
@@ -350,11 +334,6 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
     d.active = 2;   // a(x0) in the step it joins
     d.compensated = r->p.compensated ? 1 : 0;
     d.force = r->force;
-    s->ap_region[id] = s->ap_region_cap[id] = 0;
-    if (ap0 >= 0) {
-      NB_TRY(ap_place(s, r, ap0, ap_len));
-      s->ap_kept += r->ap_least;
-    }
     for (int b = 0; b < nb32; ++b) s->blk[b0 + b] = id;
     s->table_dirty = true;
     s->running.push_back(r);
@@ -394,6 +373,7 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
       NB_CUDA(cudaMemcpyAsync((void*)s->e.runs, s->plan.runs.data(),
                               sizeof(BuildRun) * s->plan.runs.size(),
                               cudaMemcpyHostToDevice, s->stream));
+    NB_TRY(ap_layout(s));
     int too_small = 0;
     plan_ens_allpairs(s->sims.data(), nsims, s->ap_region.data(), s->ap,
                       s->ap_region_cap.data(), &too_small);
@@ -490,7 +470,7 @@ int engine_iteration(nb_server* s, std::unique_lock<std::mutex>& lk) {
                             cudaMemcpyDeviceToHost, s->stream));
     NB_CUDA(cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming));
     NB_CUDA(cudaEventRecord(r->done_ev, s->stream));
-    if (r->ap_chunk >= 0) s->ap_kept -= r->ap_least;
+    s->ap_kept -= r->ap_least;
     s->finishing.push_back(r);
     s->running.erase(s->running.begin() + k);
   }
@@ -547,11 +527,11 @@ int nb_server_create(size_t hbm_budget_bytes, int max_sims, nb_server** out) {
   s->budget = hbm_budget_bytes;
   s->cap_slots = (int)slots;
   s->max_sims = max_sims;
-  s->ap_chunks = (int)std::min<size_t>(ap_bytes / (16 * kApChunk), (size_t)1 << 30);
+  s->ap_chunks = ap_bytes / (16 * kApChunk);
   int rc = NB_OK;
   do {
     EnsArgs& e = s->e;
-    if ((rc = srv_alloc(s, &s->d_ap_pool, (size_t)s->ap_chunks * kApChunk)) != NB_OK) break;
+    if ((rc = srv_alloc(s, &s->d_ap_pool, s->ap_chunks * kApChunk)) != NB_OK) break;
     s->ap.d_pool = s->d_ap_pool;
     if ((rc = srv_alloc(s, &s->ap.d_args, (size_t)max_sims)) != NB_OK) break;
     if ((rc = srv_alloc(s, &s->ap.d_src_off, (size_t)max_sims)) != NB_OK) break;
@@ -639,7 +619,6 @@ int nb_server_create(size_t hbm_budget_bytes, int max_sims, nb_server** out) {
   s->ap_region_cap.assign(max_sims, 0);
   s->blk.assign(s->cap_slots / 32, -1);
   s->free_blocks[0] = s->cap_slots / 32;
-  if (s->ap_chunks > 0) s->ap_free[0] = s->ap_chunks;
   for (int id = max_sims - 1; id >= 0; --id) s->free_ids.push_back(id);
   s->t_start = now_s();
   int dev = 0;
@@ -706,7 +685,7 @@ int nb_server_submit(nb_server* s, int n, const float* pos4, const float* vel4,
   if ((size_t)(n + 31) / 32 * 32 > (size_t)s->cap_slots)
     return set_error(NB_ERR_NOMEM, "request larger than the server's HBM budget");
   const int force = resolve_force_batch(p->force, n, p->theta);
-  if (force == NB_FORCE_NAIVE && ap_chunks_of(n) > s->ap_chunks)
+  if (force == NB_FORCE_NAIVE && ap_chunks_of(ap_region_f4(n)) > s->ap_chunks)
     return set_error(NB_ERR_NOMEM, "all-pairs request larger than the server's "
                                    "all-pairs scratch (1/8 of the HBM budget)");
   if (dump_every > 0 && n > s->frame_cap)

@@ -223,3 +223,17 @@ def test_batch_tables_that_cannot_be_had(monkeypatch):
                 assert np.array_equal(p, ref[s][0]) and np.array_equal(v, ref[s][1])
     finally:
         api.tune_set(base)
+
+
+def test_batch_above_one_gib_of_tables_takes_few_passes():
+    """524,288 particles have 128 rows of tiles and tables of 3.2 GB; 1 GiB holds
+    42 rows."""
+    base = api.tune_get()
+    t = L.nb_tune_table()
+    L.check(L.load().nb_tune_defaults(ctypes.byref(t)))
+    try:
+        L.check(L.load().nb_tune_set(ctypes.byref(t)))
+        with Ensemble([ic.two_disks(524_288, seed=3)], PRM) as ens:
+            assert ens.kernels_per_step() == 1 + 2 * 4
+    finally:
+        api.tune_set(base)

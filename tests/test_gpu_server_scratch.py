@@ -66,3 +66,24 @@ def test_whole_tables_do_not_keep_requests_out(table):
         q, w = _alone(pos, vel, steps)
         for p, v in got[k::4]:
             assert np.array_equal(p, q) and np.array_equal(v, w)
+
+
+def test_regions_move_as_requests_come_and_go(table):
+    """Requests of all three all-pairs kernels and of different lengths over a pool
+    that cannot hold their whole tables: each one's region grows, shrinks and moves
+    between steps (the second packed one when the first has gone)."""
+    t = L.nb_tune_table()
+    L.check(L.load().nb_tune_defaults(ctypes.byref(t)))
+    L.check(L.load().nb_tune_set(ctypes.byref(t)))
+    work = [((1 << 20) + 1, 1), ((1 << 20) + 31, 3), (70_001, 5), (9000, 4), (20_001, 2),
+            (1500, 5)]
+    states = [ic.two_disks(n, seed=n) for n, _ in work]
+    with Server(hbm_budget_bytes=1 << 30, max_sims=8) as srv:
+        ids = [srv.submit(*s, PRM, k) for s, (_, k) in zip(states, work)]
+        got = []
+        for rid in ids:
+            srv.wait(rid, 120)
+            got.append(srv.result(rid))
+    for (pos, vel), (_, k), (p, v) in zip(states, work, got):
+        q, w = _alone(pos, vel, k)
+        assert np.array_equal(p, q) and np.array_equal(v, w)
