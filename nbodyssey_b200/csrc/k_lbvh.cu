@@ -447,12 +447,11 @@ int launch_sort(Workspace& w, const StepArgs& a, cudaStream_t st) {
 // the keys, the permutation and the gathered positions to global memory.  The
 // same stable sort, so the same permutation.
 //
-// Bound: latency.  Up to about 100,000 keys a onesweep pass takes 9 us whatever
+// Bound: latency.  Up to about 100,000 keys a onesweep pass takes 7 us whatever
 // n is (launch, ticket, look-back); here a pass is two cluster barriers (0.5 us
-// each), and the rank and scatter of n / 16 keys per SM: 19 us for the keys and
-// four passes at n = 4,096 against 42, 25 against 47 at 20,011, 39 against 41 at
-// 65,536.  512 threads: with 1,024 the barriers cost more than the wider rank
-// gains.
+// each), and the rank and scatter of n / 16 keys per SM.  The times are at
+// sort_in_cluster.  512 threads: with 1,024 the barriers cost more than the wider
+// rank gains.
 // ---------------------------------------------------------------------------
 constexpr int kClusterCtas = 16;
 constexpr int kClusterThreads = 512;
@@ -779,10 +778,14 @@ static bool cluster_sort_fits() {
   return known[dev] == 1;
 }
 
-// Keys and sort, one launch against Morton kernel and onesweep passes: 30 bits
-// 24 / 34 us at n = 10,000, 34 / 40 at 40,000, equal at 65,536; 63 bits 42 / 60 at
-// 10,000, 58 / 65 at 30,000, equal at 40,000 (8 passes over n / 16 keys per SM, while
-// the onesweep's grow little with n).
+// Box, keys and sort, one launch against prep, Morton kernel and onesweep passes
+// (phase events of a force call, which add about 3 us to each phase, empty ones
+// included): 30 bits 27 / 41 us at n = 4,096, 32 / 49 at 20,011, 39 / 49 at 40,000, 47 /
+// 52 at 65,536, all that fits; 63 bits 47 / 70 at 10,000, 64 / 76 at 30,000, 70 / 77 at
+// 36,864, 72 / 77 at 40,000, 80 / 79 at 50,000 (8 passes over n / 16 keys per SM, while
+// the onesweep's grow little with n).  Whole calls back to back: 162 / 175 us at 20,011
+// particles, 283 / 293 at 65,536; with 63 bits 219 / 241 at 30,000 and equal at 36,864
+// (252 / 251), where the line is.
 bool sort_in_cluster(int n, int key_bits) {
   if (n > (key_bits == 63 ? kClusterMax / 16 * 9 : kClusterMax)) return false;
   return key_bits == 63 ? cluster_sort_fits<uint64_t>() : cluster_sort_fits<uint32_t>();

@@ -14,8 +14,8 @@
 //   1e-5 relative margin, far above the few-ulp rounding of the exact test);
 // * warp semantics: otherwise the group's target furthest out in the direction
 //   of the child's octant (seen from the box centre) is tested exactly, and its
-//   rejection opens the child; it settles 961 of the 1,083 opened children per
-//   warp at 1M particles (the extreme along the dominant axis, 918, and takes
+//   rejection opens the child; it settles 944 of the 1,068 opened children per
+//   warp at 1M particles (the extreme along the dominant axis, 906, and takes
 //   twice the instructions to pick);
 // * thread semantics: a child that even the farthest box point rejects is
 //   rejected by every target;

@@ -1,6 +1,8 @@
-// Autotuner: per device, the all-pairs launch shape per size, the Barnes-Hut
-// walk's warps per block and the all-pairs / Barnes-Hut crossover that
-// NB_FORCE_AUTO uses, measured on the device itself.
+// Autotuner: per device, the launch shape per size of the tiled all-pairs kernel
+// (which runs above 2^20 particles; smaller calls take kernels whose shapes follow
+// from n alone), the Barnes-Hut walk's warps per block for launches of more than
+// 48 warps per SM, and the all-pairs / Barnes-Hut crossover that NB_FORCE_AUTO
+// uses, measured on the device itself.
 //
 // The reference has one fixed shape (kForceBlock = 256, src/forces.cuh:25)
 // and a force module the user picks by hand (src/forces.cu:68-86).  Here the
@@ -12,7 +14,7 @@
 // events on a private stream, best of three after a warm-up.
 //
 // The shape decides only the launch: the per-target summation order of the
-// all-pairs kernel depends on the source chunking alone, so two runs with the
+// tiled kernel depends on the source chunking alone, so two runs with the
 // same table give the same bits, whether the table was measured, loaded or
 // set by hand (nb_tune_set).
 #include <sys/stat.h>
