@@ -17,6 +17,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "f32x2.cuh"
 #include "nb_internal.cuh"
@@ -574,12 +575,14 @@ int launch_ens_allpairs(const EnsArgs& e, const EnsAllPairs& ap, cudaStream_t st
 // Energy.  PE = -G sum_{i<j} m_i m_j rsqrt(r_ij^2 + eps^2), each unordered pair
 // once.  A CTA holds a tile of kEThreads x K particles (K per thread) and runs
 // over its chunk of the partners from the tile's own start on: partners past
-// the tile count once; the tile's own particles are summed in both orders with
-// the self term, so that part is halved and the self term (the same float
-// rsqrt(eps^2) the loop used) removed.  Pair math in FP32, two partners per
-// packed instruction; each 256-partner sum is added in FP64, and KE, PE and
-// momentum are reduced in FP64 in a fixed order (block partials, then the last
-// block).
+// the tile count once; the tile's own particles are summed in both orders, so
+// that part is halved, a particle's own mass taken as 0.  (A self term summed with
+// the others and removed again costs their low bits: with a body of 10^6 times the
+// others' mass PE was 16 % off at n = 513 and 0.4 % at 2,560, now 2e-7; 16,384
+// particles 83.5 -> 84.5 us, 100,000 1,424 -> 1,430.)
+// Pair math in FP32, two partners per packed instruction; each 256-partner sum
+// is added in FP64, and KE, PE and momentum are reduced in FP64 in a fixed order
+// (block partials, then the last block).
 //
 // Bound: 7 packed FP32 operations, 2 scalar ones and 2 MUFU rsqrt per two pairs,
 // which fill the FMA pipe (64 packed lanes a cycle and SM) and the MUFU unit (16)
@@ -591,8 +594,10 @@ constexpr int kEThreads = 128;
 constexpr int kETile = 256;      // partners staged together
 constexpr int kEReduceThreads = 256;
 
+// Wide tiles: 7 CTAs per SM (72 registers); with 8 the CTAs of n = 20,011, fewer
+// than fit at once, lie less evenly over the SMs: 118 us a call against 107.
 template <int K>
-__global__ void __launch_bounds__(kEThreads) k_energy_pairs(
+__global__ void __launch_bounds__(kEThreads, K == 4 ? 7 : 16) k_energy_pairs(
     const float4* __restrict__ pos, int n, float eps2, int jchunk,
     double* __restrict__ pe_part) {
   __shared__ __align__(16) float s_src[kETile * 4];   // (x0,x1,y0,y1)(z0,z1,m0,m1) pairs
@@ -603,7 +608,7 @@ __global__ void __launch_bounds__(kEThreads) k_energy_pairs(
   const int j1 = min((int)(blockIdx.y + 1) * jchunk, n);
   const int j0 = max((int)blockIdx.y * jchunk, i0);   // T is a multiple of kETile or divides it
   f2 nx[K], ny[K], nz[K];
-  double once[K], own[K];
+  double sum[K];   // of m_j / r
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int i = i0 + k * kEThreads + tid;
@@ -611,12 +616,11 @@ __global__ void __launch_bounds__(kEThreads) k_energy_pairs(
     nx[k] = pk2(-p.x, -p.x);
     ny[k] = pk2(-p.y, -p.y);
     nz[k] = pk2(-p.z, -p.z);
-    once[k] = own[k] = 0.0;
+    sum[k] = 0.0;
   }
   const f2 e2 = pk2(eps2, eps2);
-  for (int jt = j0; jt < j1;) {
-    // a stage never mixes the tile's own particles with later ones
-    const int je = min(jt < i0 + T ? min(jt + kETile, i0 + T) : jt + kETile, j1);
+  // partners [jt, je) of at most kETile, a particle's own mass as 0 where `own`
+  auto stage = [&](int jt, int je, auto own) {
     __syncthreads();   // the previous stage has been read
     for (int k = tid; k < kETile; k += kEThreads) {
       const float4 p = jt + k < je ? pos[jt + k] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -629,46 +633,59 @@ __global__ void __launch_bounds__(kEThreads) k_energy_pairs(
     for (int k = 0; k < K; ++k) acc[k] = 0.f;
     const int pairs = (je - jt + 1) >> 1;
     const ulonglong2* src = reinterpret_cast<const ulonglong2*>(s_src);
+    const int at = i0 + tid - jt;   // where the stage holds the first own particle
+    auto run = [&](int q0, int q1, auto masked) {
 #pragma unroll 4
-    for (int q = 0; q < pairs; ++q) {
-      const ulonglong2 A = src[2 * q], B = src[2 * q + 1];
+      for (int q = q0; q < q1; ++q) {
+        const ulonglong2 A = src[2 * q], B = src[2 * q + 1];
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const f2 dx = add2(A.x, nx[k]), dy = add2(A.y, ny[k]), dz = add2(B.x, nz[k]);
-        // eps^2 last: seeding the chain with it saves an instruction but
-        // shifts the sum's rounding bias (2e-9 of PE at n = 100,000)
-        const f2 r2 = add2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), e2);
-        float r0, r1;
-        up2(r2, r0, r1);
-        // one chain over a stage's partners in order: two packed chains take
-        // 3 % less time, but their sums round 2 to 4e-10 of PE away from it
-        float m0, m1;
-        up2(B.y, m0, m1);
-        acc[k] = __fmaf_rn(m0, mufu_rsqrt(r0), acc[k]);
-        acc[k] = __fmaf_rn(m1, mufu_rsqrt(r1), acc[k]);
+        for (int k = 0; k < K; ++k) {
+          const f2 dx = add2(A.x, nx[k]), dy = add2(A.y, ny[k]), dz = add2(B.x, nz[k]);
+          // eps^2 last: seeding the chain with it saves an instruction but
+          // shifts the sum's rounding bias (2e-9 of PE at n = 100,000)
+          const f2 r2 = add2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), e2);
+          float r0, r1;
+          up2(r2, r0, r1);
+          // one chain over a stage's partners in order: two packed chains take
+          // 3 % less time, but their sums round 2 to 4e-10 of PE away from it
+          float m0, m1;
+          up2(B.y, m0, m1);
+          if (masked) {
+            if (2 * q == at + k * kEThreads) m0 = 0.f;
+            if (2 * q + 1 == at + k * kEThreads) m1 = 0.f;
+          }
+          acc[k] = __fmaf_rn(m0, mufu_rsqrt(r0), acc[k]);
+          acc[k] = __fmaf_rn(m1, mufu_rsqrt(r1), acc[k]);
+        }
       }
+    };
+    if (own) {
+      // a warp's own particles are 32 in a row of every kEThreads: the rest of the
+      // stage needs no look at the index
+      const int mine = (at & ~31) / 2;
+      for (int q = 0; q < pairs; q += 16) {
+        const int end = min(q + 16, pairs);
+        if (((q - mine) & (kEThreads / 2 - 1)) == 0) run(q, end, std::true_type{});
+        else run(q, end, std::false_type{});
+      }
+    } else {
+      run(0, pairs, std::false_type{});
     }
-    const bool mine = jt < i0 + T;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const double s = (double)acc[k];
-      if (mine) own[k] += s;
-      else once[k] += s;
-    }
-    jt = je;
-  }
-  // the chunk that starts this tile's run over its own particles removes the
-  // self terms
-  const bool self = j0 == i0 && j0 < j1;
-  const float self_inv = mufu_rsqrt(eps2);
+    for (int k = 0; k < K; ++k) sum[k] += (double)acc[k];
+  };
+  const int mid = min(i0 + T, j1);
+  for (int jt = j0; jt < mid; jt += kETile) stage(jt, min(jt + kETile, mid), std::true_type{});
+#pragma unroll
+  for (int k = 0; k < K; ++k) sum[k] *= 0.5;
+  for (int jt = max(j0, i0 + T); jt < j1; jt += kETile)
+    stage(jt, min(jt + kETile, j1), std::false_type{});
   double pe = 0.0;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int i = i0 + k * kEThreads + tid;
     if (i >= n) continue;
-    const float m = pos[i].w;
-    const double s = self ? (double)__fmul_rn(m, self_inv) : 0.0;
-    pe += (double)m * (once[k] + 0.5 * (own[k] - s));
+    pe += (double)pos[i].w * sum[k];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) pe += __shfl_down_sync(0xffffffffu, pe, o);

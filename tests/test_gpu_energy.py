@@ -30,3 +30,20 @@ def test_energy_vs_fp64(n):
     assert abs(e - (ke + pe)) <= 1e-12 * (abs(ke) + abs(pe))
     if n == 1:
         assert pe == 0.0
+
+
+@pytest.mark.parametrize("eps", [0.05, 1e-4])
+@pytest.mark.parametrize("n,where", [(129, 0), (513, 512), (1000, 500), (2560, 2559),
+                                     (16384, 8192), (20011, 20010)])
+def test_energy_with_a_dominant_body(n, where, eps):
+    """A central body of 10^6 times the others' mass: its self term would be far
+    larger than the sum of the others' terms in its potential."""
+    pos, vel = ic.two_disks(n, seed=n)
+    pos[where, 3] *= np.float32(1e6)
+    with api.Simulation(pos, vel, api.SimParams(epsilon=eps, force="naive")) as sim:
+        _, _, pe = sim.energy()
+    ref = O.energy_f64(pos, vel, eps)[2]
+    # as above, but every FP32 sum holds terms of the potential alone; close
+    # pairs at small eps: each r^2 is of differences exact to 2^-24 of themselves
+    rel = 2.0 ** -22 + 259 * 2.0 ** -24
+    assert abs(pe - ref) <= rel * abs(ref)
