@@ -241,7 +241,7 @@ NB_API int nb_record(nb_sim* s, int slot /* 0..15 */);
 NB_API int nb_elapsed_ms(nb_sim* s, int slot0, int slot1, double* ms);
 
 /* Use a captured CUDA graph for each step (default on).  The graph is
- * re-captured when the parameters change. */
+ * re-captured when the parameters change or scratch that it uses has moved. */
 NB_API int nb_set_graphs(nb_sim* s, int enable);
 /* Enqueues a write of `bytes` (>= the 126 MB L2) to a scratch buffer on the
  * simulation's stream, evicting the state from L2 between timed steps. */
@@ -275,7 +275,11 @@ NB_API int nb_compare_forces(nb_sim* s, double* max_rel, double* mean_rel);
  * on caller-owned device arrays (float4 rows) on a caller-given stream
  * (cudaStream_t passed as void*; NULL = legacy default stream).  Scratch is
  * held by a workspace (the reference's process-global Scratch,
- * src/forces_bh.cu:50-69), grown only when n grows.
+ * src/forces_bh.cu:50-69), grown only when n grows; under stream capture it
+ * cannot grow, so its largest n runs once before.  All-pairs calls of 2,560 to
+ * 2^20 particles hold up to 1 GiB (118 MB at 50,001 particles, 805 MB at
+ * 262,144), less with the same results where that cannot be had or the
+ * environment variable NBODY_B200_ALLPAIRS_MIB bounds it.
  * ==================================================================== */
 typedef struct nb_workspace nb_workspace;
 NB_API int nb_workspace_create(nb_workspace** out);
