@@ -154,7 +154,8 @@ int ws_reserve(Workspace& w, int n, int key_bits) {
   NB_CUDA(cudaMemset(w.nodes, 0, ni * sizeof(Node)));
   NB_CUDA(cudaMemset(w.pairs, 0, (size_t)cap * sizeof(PairRec)));
   w.status_tiles = sort_status_tiles(cap);
-  size_t words = 8 * kSortRadix + 8 + (size_t)8 * w.status_tiles * kSortRadix;
+  // look-back words of the passes that keys of kb bits take
+  size_t words = 8 * kSortRadix + 8 + (size_t)(kb == 63 ? 8 : 4) * w.status_tiles * kSortRadix;
   // the sort's words and the build's segments in one allocation: each takes about
   // 0.3 ms of a first call from 1 MB on, whatever its size
   static_assert(kSortRadix % 2 == 0, "the segments are 8-byte aligned");
